@@ -64,7 +64,8 @@ struct Split {
     double* gram;            // [nb][gstride]
     double* coef;            // [nb][cstride]
     double* usc;             // [nb][dim][maxk] scaled offsets u = x_pq / eps of every row
-    int64_t ustride;         // dim * maxk
+    int64_t ustride;         // dim * maxk (+ maxk with vjp: E of every row)
+    bool vjp;                // position VJP: column E c of B, two right-hand sides (b~, s) per group
     int maxk;
     int32_t* gst;            // [nb] group status words
     // tensor-core Gram (DCPSE_ASSEMBLE_TC): B of every particle of the batch
@@ -157,7 +158,10 @@ __global__ void __launch_bounds__(256) eps_kernel(AsmArgs a, Split S, int64_t b0
 }
 
 // ---------------------------------------------------------------- 1. Gram --
-template <int DIM, int NPP>
+// VJP: B has one more column, E_q (f_q - f_p), and the entries (i, nu) after
+// the Gram entries are s = sum_q omega_q (f_q - f_p) v_q; E_q of every row is
+// kept beside u for the chain rule.
+template <int DIM, int NPP, bool VJP>
 __global__ void __launch_bounds__(256) gram_kernel(AsmArgs a, Split S, int64_t b0, int64_t b1) {
     extern __shared__ double smem[];
     __shared__ ProgShared P;
@@ -168,7 +172,7 @@ __global__ void __launch_bounds__(256) gram_kernel(AsmArgs a, Split S, int64_t b
     double* Bs = smem + (size_t)wib * (kCh * S.ldb + S.nslots * 32);
     double* V = Bs + kCh * S.ldb;
     const int nu = T.nu;
-    const int npairs = T.npairs;
+    const int npairs = T.npairs + (VJP ? nu : 0);
     const int ngroups = T.ngroups;
     const int nprog = T.nprog;
 
@@ -177,8 +181,8 @@ __global__ void __launch_bounds__(256) gram_kernel(AsmArgs a, Split S, int64_t b
 #pragma unroll
     for (int t = 0; t < NPP; ++t) {
         int e = t * 32 + lane;
-        pi[t] = (e < npairs) ? T.pi[e] : 0;
-        pj[t] = (e < npairs) ? T.pj[e] : 0;
+        pi[t] = (e < T.npairs) ? T.pi[e] : ((VJP && e < npairs) ? e - T.npairs : 0);
+        pj[t] = (e < T.npairs) ? T.pj[e] : ((VJP && e < npairs) ? nu : 0);
     }
 
     const int wpc = blockDim.x >> 5;
@@ -215,6 +219,10 @@ __global__ void __launch_bounds__(256) gram_kernel(AsmArgs a, Split S, int64_t b
                 const double E = cw_exp(-norm2<DIM>(o) / (2.0 * eps * eps));
                 monomials<DIM>(u, V, P, nprog, lane);
                 for (int j = 0; j < nu; ++j) Bs[lane * S.ldb + j] = E * V[P.uslot[j] * 32 + lane];
+                if constexpr (VJP) {
+                    Ur[DIM * S.maxk + q] = E;
+                    Bs[lane * S.ldb + nu] = E * (a.f[a.cols[beg + q]] - a.f[p]);
+                }
             }
             __syncwarp();
             for (int r = 0; r < cnt; ++r) {
@@ -233,6 +241,7 @@ __global__ void __launch_bounds__(256) gram_kernel(AsmArgs a, Split S, int64_t b
 }
 
 #include "dcpse_gram_tc.cuh"
+#include "dcpse_vjp.cuh"
 
 // Gram kernel for bases whose entries do not fit in the lanes' registers
 // (more than 40 x 32 pairs, e.g. 7260 for the 120-function basis of
@@ -373,7 +382,7 @@ __global__ void __launch_bounds__(256) gram_b_kernel(AsmArgs a, Split S, int64_t
 // down (or that was not assembled) keeps running on its own work space and
 // only its stores are suppressed.
 template <int LPP>
-__global__ void __launch_bounds__(kQrWarps * 32) qr_kernel(AsmArgs a, Split S, int64_t nb) {
+__global__ void __launch_bounds__(kQrWarps * 32) qr_kernel(AsmArgs a, Split S, int64_t b0, int64_t nb) {
     constexpr int PPW = 32 / LPP;
     extern __shared__ double smem[];
     const AsmTables& T = *a.tab;
@@ -412,6 +421,14 @@ __global__ void __launch_bounds__(kQrWarps * 32) qr_kernel(AsmArgs a, Split S, i
                     if (j < n) {
                         const int ui = T.gidx[g][i], uj = T.gidx[g][j];
                         v = G[T.upair[min(ui, uj)][max(ui, uj)]];
+                    } else if (S.vjp) {
+                        // b~ = sum_o gbar_o b_o, then s
+                        if (j == n) {
+                            for (int r = 0; r < T.nout_rhs[g]; ++r)
+                                v += a.gbar[(int64_t)T.out_of_rhs[g][r] * a.n + b0 + slot] * T.b_out[g][r][i];
+                        } else {
+                            v = G[S.npairs + T.gidx[g][i]];
+                        }
                     } else {
                         v = fast ? T.b_out[g][j - n][i] : T.b_term[g][j - n][i];
                     }
@@ -668,7 +685,7 @@ cudaError_t launch_eps(const AsmArgs& a, const Split& S, int64_t b0, int64_t b1,
     return cudaGetLastError();
 }
 
-template <int DIM, int NPP>
+template <int DIM, int NPP, bool VJP>
 cudaError_t launch_gram(const AsmArgs& a, const Split& S, int64_t b0, int64_t b1, cudaStream_t s) {
     int warps = warps_of(a);
     const size_t per_warp = (size_t)(kCh * S.ldb + S.nslots * 32) * sizeof(double);
@@ -685,7 +702,7 @@ cudaError_t launch_gram(const AsmArgs& a, const Split& S, int64_t b0, int64_t b1
         return cudaGetLastError();
     }
     const size_t bytes = per_warp * warps;
-    auto kern = gram_kernel<DIM, NPP == 0 ? 1 : NPP>;
+    auto kern = gram_kernel<DIM, NPP == 0 ? 1 : NPP, VJP>;
     int grid = 0;
     cudaError_t e = persistent(kern, warps * 32, bytes, warps, b1 - b0, grid);
     if (e != cudaSuccess) return e;
@@ -707,12 +724,12 @@ size_t qr_bytes(const Split& S, int lpp) {
 constexpr int kQrGlobalPerSm = 4;
 
 template <int LPP>
-cudaError_t launch_qr(const AsmArgs& a, Split S, int64_t nb, cudaStream_t s) {
+cudaError_t launch_qr(const AsmArgs& a, Split S, int64_t b0, int64_t nb, cudaStream_t s) {
     constexpr int PPW = 32 / LPP;
     S.pstride = qr_pstride(S, LPP);
     if (S.qws) {
         const int64_t grid = std::min<int64_t>((int64_t)num_sms() * kQrGlobalPerSm, nb);
-        qr_kernel<LPP><<<(unsigned)std::max<int64_t>(grid, 1), 32, 0, s>>>(a, S, nb);
+        qr_kernel<LPP><<<(unsigned)std::max<int64_t>(grid, 1), 32, 0, s>>>(a, S, b0, nb);
         return cudaGetLastError();
     }
     const size_t bytes = qr_bytes(S, LPP);
@@ -720,7 +737,7 @@ cudaError_t launch_qr(const AsmArgs& a, Split S, int64_t nb, cudaStream_t s) {
     int grid = 0;
     cudaError_t e = persistent(kern, kQrWarps * 32, bytes, (int64_t)kQrWarps * PPW, nb, grid);
     if (e != cudaSuccess) return e;
-    kern<<<grid, kQrWarps * 32, bytes, s>>>(a, S, nb);
+    kern<<<grid, kQrWarps * 32, bytes, s>>>(a, S, b0, nb);
     return cudaGetLastError();
 }
 
@@ -754,14 +771,14 @@ int qr_lanes_auto(const Split& S) {
     return 32;
 }
 
-cudaError_t launch_qr_any(const AsmArgs& a, const Split& S, int lpp, int64_t nb, cudaStream_t s) {
+cudaError_t launch_qr_any(const AsmArgs& a, const Split& S, int lpp, int64_t b0, int64_t nb, cudaStream_t s) {
     switch (lpp) {
-        case 1: return launch_qr<1>(a, S, nb, s);
-        case 2: return launch_qr<2>(a, S, nb, s);
-        case 4: return launch_qr<4>(a, S, nb, s);
-        case 8: return launch_qr<8>(a, S, nb, s);
-        case 16: return launch_qr<16>(a, S, nb, s);
-        default: return launch_qr<32>(a, S, nb, s);
+        case 1: return launch_qr<1>(a, S, b0, nb, s);
+        case 2: return launch_qr<2>(a, S, b0, nb, s);
+        case 4: return launch_qr<4>(a, S, b0, nb, s);
+        case 8: return launch_qr<8>(a, S, b0, nb, s);
+        case 16: return launch_qr<16>(a, S, b0, nb, s);
+        default: return launch_qr<32>(a, S, b0, nb, s);
     }
 }
 
@@ -794,8 +811,8 @@ cudaError_t run(const AsmArgs& a, const AsmTables& h, const Split& S, int lpp, c
         const int64_t b1 = std::min(a.n, b0 + a.scratch_particles);
         cudaError_t e = launch_eps<DIM>(a, S, b0, b1, s);
         if (e == cudaSuccess)
-            e = S.tc ? launch_gram_tc<DIM>(a, S, b0, b1, s) : launch_gram<DIM, NPP>(a, S, b0, b1, s);
-        if (e == cudaSuccess) e = launch_qr_any(a, S, lpp, b1 - b0, s);
+            e = S.tc ? launch_gram_tc<DIM>(a, S, b0, b1, s) : launch_gram<DIM, NPP, false>(a, S, b0, b1, s);
+        if (e == cudaSuccess) e = launch_qr_any(a, S, lpp, b0, b1 - b0, s);
         if (e == cudaSuccess) e = launch_weights<DIM>(a, S, b0, b1, s);
         if (e != cudaSuccess) return e;
     }
@@ -816,23 +833,54 @@ cudaError_t dispatch(const AsmArgs& a, const AsmTables& h, const Split& S, int l
     return run<DIM, 0>(a, h, S, lpp, s);  // the wide Gram kernel
 }
 
-Split make_split(const AsmTables& h, int flags) {
+template <int DIM>
+cudaError_t launch_chain(const AsmArgs& a, const Split& S, int ngroups, int64_t b0, int64_t b1, cudaStream_t s) {
+    const int warps = warps_of(a);
+    const size_t bytes = (size_t)(S.cstride + (S.nslots + 2 * ngroups) * 32) * sizeof(double) * warps;
+    auto kern = vjp_chain_kernel<DIM>;
+    int grid = 0;
+    cudaError_t e = persistent(kern, warps * 32, bytes, warps, b1 - b0, grid);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, warps * 32, bytes, s>>>(a, S, b0, b1);
+    return cudaGetLastError();
+}
+
+template <int DIM>
+cudaError_t vjp_run(const AsmArgs& a, const AsmTables& h, const Split& S, int lpp, cudaStream_t s) {
+    const int npp = (h.npairs + h.nu + 31) / 32;
+    for (int64_t b0 = 0; b0 < a.n; b0 += a.scratch_particles) {
+        const int64_t b1 = std::min(a.n, b0 + a.scratch_particles);
+        cudaError_t e = launch_eps<DIM>(a, S, b0, b1, s);
+        if (e == cudaSuccess)
+            e = npp <= 2   ? launch_gram<DIM, 2, true>(a, S, b0, b1, s)
+                : npp <= 7 ? launch_gram<DIM, 7, true>(a, S, b0, b1, s)
+                : npp <= 8 ? launch_gram<DIM, 8, true>(a, S, b0, b1, s)
+                           : launch_gram<DIM, 40, true>(a, S, b0, b1, s);
+        if (e == cudaSuccess) e = launch_qr_any(a, S, lpp, b0, b1 - b0, s);
+        if (e == cudaSuccess) e = launch_chain<DIM>(a, S, h.ngroups, b0, b1, s);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+Split make_split(const AsmTables& h, int flags, bool vjp = false) {
     Split S{};
     const bool fast = (flags & DCPSE_ASSEMBLE_FAST_FLAG) != 0;
-    S.gstride = (h.npairs + 1) & ~1;
+    S.vjp = vjp;
+    S.gstride = (h.npairs + (vjp ? h.nu : 0) + 1) & ~1;
     S.nmax = 1;
     S.qwords = 1;
     int off = 0;
     for (int g = 0; g < h.ngroups; ++g) {
         const int n = h.gn[g];
-        S.nrhs[g] = fast ? h.nout_rhs[g] : h.nterm_rhs[g];
+        S.nrhs[g] = vjp ? 2 : (fast ? h.nout_rhs[g] : h.nterm_rhs[g]);
         S.c_off[g] = off;
         off += n * S.nrhs[g];
         S.nmax = std::max(S.nmax, n);
         S.qwords = std::max(S.qwords, n * (n + S.nrhs[g]) + n * S.nrhs[g]);
     }
     S.cstride = (off + 1) & ~1;
-    S.ldb = h.nu | 1;
+    S.ldb = (h.nu + (vjp ? 1 : 0)) | 1;
     S.nslots = h.nslots;
     S.nout = h.noutputs;
     S.npairs = h.npairs;
@@ -858,6 +906,12 @@ int64_t assembly_scratch_bytes(const AsmTables& h, int flags, int maxk) {
     if (assembly_uses_tc(h, flags, maxk))
         b += (int64_t)h.nu * tc_kpad(maxk) * (int64_t)sizeof(double) + 32 * (int64_t)sizeof(int32_t);
     return b;
+}
+
+int64_t vjp_scratch_bytes(const AsmTables& h, int maxk) {
+    const Split S = make_split(h, DCPSE_ASSEMBLE_FAST_FLAG, true);
+    return (int64_t)(S.gstride + S.cstride + (int64_t)(h.dim + 1) * std::max(maxk, 1)) * (int64_t)sizeof(double) +
+           (int64_t)sizeof(int32_t);
 }
 
 int64_t assembly_qr_ws_bytes(const AsmTables& h, int flags) {
@@ -937,6 +991,26 @@ cudaError_t assemble(const AsmArgs& a, const AsmTables& h, cudaStream_t s) {
     if (h.dim == 3) return dispatch<3>(a, h, S, lpp, s);
     if (h.dim == 2) return dispatch<2>(a, h, S, lpp, s);
     return dispatch<1>(a, h, S, lpp, s);
+}
+
+cudaError_t vjp_entries(const AsmArgs& a, const AsmTables& h, cudaStream_t s) {
+    if (a.n == 0) return cudaSuccess;
+    if (!a.scratch || a.scratch_particles < 1) return cudaErrorInvalidValue;
+    Split S = make_split(h, DCPSE_ASSEMBLE_FAST_FLAG, true);
+    const int64_t nb = a.scratch_particles;
+    S.gram = a.scratch;
+    S.coef = S.gram + nb * S.gstride;
+    S.maxk = std::max(a.maxk, 1);
+    S.ustride = (int64_t)(h.dim + 1) * S.maxk;
+    S.usc = S.coef + nb * S.cstride;
+    S.gst = reinterpret_cast<int32_t*>(S.usc + nb * S.ustride);
+    int lpp = a.qr_lanes;
+    if (lpp != 1 && lpp != 2 && lpp != 4 && lpp != 8 && lpp != 16 && lpp != 32) lpp = qr_lanes_auto(S);
+    if (qr_bytes(S, lpp) > (size_t)smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024))
+        lpp = 32;  // a lane grouping chosen for the assembly's right-hand sides
+    if (h.dim == 3) return vjp_run<3>(a, h, S, lpp, s);
+    if (h.dim == 2) return vjp_run<2>(a, h, S, lpp, s);
+    return vjp_run<1>(a, h, S, lpp, s);
 }
 
 }  // namespace dcpse

@@ -294,6 +294,7 @@ struct dcpse_plan_s {
     double* rowsum = nullptr;
     int rowsum_prec = -1;
     double* gentry = nullptr;
+    double* vjp_eps = nullptr;  // eps and eps^-|alpha| of the position VJP [1 + groups][n]
     // transposed Laplacian weights of output 0 for the RK4 adjoint, and the
     // FP32 ones on a sliced ELL layout of the transposed list
     float *wT32 = nullptr, *rs32 = nullptr;
@@ -336,6 +337,7 @@ struct dcpse_plan_s {
         dfree(t_idx);
         dfree(rowsum);
         dfree(gentry);
+        dfree(vjp_eps);
         dfree(wT32);
         dfree(rs32);
         dfree(wT64);
@@ -526,6 +528,24 @@ int build_program(AsmTables* T) {
         T->uslot[j] = (unsigned char)cur;
     }
     T->nslots = dim + 1 + T->nprog;
+    // derivative monomials: a basis holds every monomial of lower degree but,
+    // for even |alpha|, the constant, whose slot is dim
+    for (int j = 0; j < T->nu; ++j)
+        for (int d = 0; d < dim; ++d) {
+            T->dslot[j][d] = (unsigned char)dim;
+            if (T->uexp[j][d] == 0) continue;
+            int e[kMaxDim] = {0, 0, 0}, deg = 0;
+            for (int c = 0; c < dim; ++c) deg += e[c] = (int)T->uexp[j][c] - (c == d);
+            for (int i = 0; i < T->nu; ++i) {
+                bool same = true;
+                for (int c = 0; c < dim; ++c) same &= (int)T->uexp[i][c] == e[c];
+                if (same) {
+                    T->dslot[j][d] = T->uslot[i];
+                    deg = 0;
+                }
+            }
+            if (deg != 0) return -1;
+        }
     return 0;
 }
 
@@ -1224,6 +1244,23 @@ int dcpse_neighbors_ptr(dcpse_plan_t* P, const int64_t** d_rowptr, const int32_t
 namespace {
 int ensure_sell(dcpse_plan_t* P);
 int ensure_sell64(dcpse_plan_t* P);
+
+// The plan's scratch for batches of particles of `per` bytes each, at most
+// kAsmScratchBytes (the Gram entries, coefficients and scaled offsets of the
+// particles in flight).
+int asm_batches(dcpse_plan_t* P, AsmArgs& a, int64_t per) {
+    const int64_t nb = std::min<int64_t>(a.n, std::max<int64_t>(4096, kAsmScratchBytes / per));
+    const int64_t bytes = nb * per + 16;
+    if (P->asm_scratch_bytes < bytes) {
+        dfree(P->asm_scratch);
+        P->asm_scratch_bytes = 0;
+        DCPSE_CK(dalloc(&P->asm_scratch, (size_t)(bytes + 7) / 8));
+        P->asm_scratch_bytes = bytes;
+    }
+    a.scratch = P->asm_scratch;
+    a.scratch_particles = nb;
+    return DCPSE_OK;
+}
 }  // namespace
 
 int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fixed, int flags) {
@@ -1297,18 +1334,7 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
     a.err = P->d_err;
     a.order = nullptr;
     if (n > 0) {
-        // batches of at most kAsmScratchBytes of scratch (Gram entries and
-        // coefficients of the particles in flight)
-        const int64_t per = assembly_scratch_bytes(*P->htab, flags, P->maxk);
-        const int64_t nb = std::min<int64_t>(n, std::max<int64_t>(4096, kAsmScratchBytes / per));
-        const int64_t bytes = nb * per + 16;
-        if (P->asm_scratch_bytes < bytes) {
-            dfree(P->asm_scratch);
-            P->asm_scratch_bytes = 0;
-            DCPSE_CK(dalloc(&P->asm_scratch, (size_t)(bytes + 7) / 8));
-            P->asm_scratch_bytes = bytes;
-        }
-        a.scratch = P->asm_scratch;
+        if (int rc = asm_batches(P, a, assembly_scratch_bytes(*P->htab, flags, P->maxk))) return rc;
         const int64_t qb = assembly_qr_ws_bytes(*P->htab, flags);
         if (qb > 0 && P->qr_ws_bytes < qb) {
             dfree(P->qr_ws);
@@ -1317,7 +1343,6 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
             P->qr_ws_bytes = qb;
         }
         a.qws = qb > 0 ? P->qr_ws : nullptr;
-        a.scratch_particles = nb;
     }
     if (P->asm_bin_width > 0 && n > 0) {
         if (!P->korder || P->korder_width != P->asm_bin_width) {
@@ -1616,20 +1641,38 @@ int dcpse_vjp_positions(dcpse_plan_t* P, const double* d_pos, const double* d_ep
         if (P->htab->gn[g] > kMaxBasisSmall)
             return fail(DCPSE_ERR_CAPACITY, "position VJP: bases of at most 35 functions");
     if (int rc = ensure_transpose(P)) return rc;
+    const int64_t n = P->n;
+    if (n == 0) return DCPSE_OK;
     if (!P->gentry) DCPSE_CK(dalloc(&P->gentry, (size_t)P->nnz * P->dim));
-    VjpArgs a{};
+    if (!P->vjp_eps) DCPSE_CK(dalloc(&P->vjp_eps, (size_t)n * (1 + P->htab->ngroups)));
+    AsmArgs a{};
     a.tab = P->dtab;
-    a.n = P->n;
-    a.pos = d_pos;
+    a.dim = P->dim;
+    a.n = n;
+    a.pos = a.spos = d_pos;
     a.rowptr = P->rowptr;
     a.cols = P->cols;
     a.geom = plan_geom(P);
     a.h_over_eps = P->hoe;
     a.eps_fixed = d_eps_fixed;
+    a.flags = DCPSE_ASSEMBLE_FAST;
+    a.eps = P->vjp_eps;
+    a.eip_group = P->vjp_eps + n;
+    a.nnz = P->nnz;
+    a.warps = P->asm_warps;
+    a.qr_lanes = P->asm_qr_lanes;
+    a.maxk = P->maxk;
+    a.err = P->d_err;
     a.f = d_f;
     a.gbar = d_g;
     a.gentry = P->gentry;
-    DCPSE_CK(vjp_positions(a, *P->htab, P->t_row, P->t_idx, d_grad, P->stream));
+    a.gown = d_grad;
+    if (int rc = asm_batches(P, a, vjp_scratch_bytes(*P->htab, P->maxk))) return rc;
+    cudaError_t e = vjp_entries(a, *P->htab, P->stream);
+    if (e == cudaErrorInvalidConfiguration)
+        return fail(DCPSE_ERR_CAPACITY, "position VJP: the QR work space of this lane grouping exceeds shared memory");
+    DCPSE_CK(e);
+    DCPSE_CK(vjp_gather(P->t_row, P->t_idx, n, P->dim, P->gentry, d_grad, P->stream));
     return DCPSE_OK;
 }
 

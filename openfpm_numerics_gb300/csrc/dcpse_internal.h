@@ -119,6 +119,10 @@ struct AsmTables {
     int nslots;
     unsigned char prog[kMaxSlots][2];
     unsigned char uslot[kMaxUnion];              // slot holding union monomial j
+    // slot of union monomial j with its exponent along d lowered by one (the
+    // monomial of d m_j / d u_d, before the factor uexp[j][d]); the constant's
+    // slot dim also where the exponent is 0
+    unsigned char dslot[kMaxUnion][kMaxDim];
 };
 
 struct AsmArgs {
@@ -151,6 +155,12 @@ struct AsmArgs {
     int64_t scratch_particles;  // batch size the scratch holds
     int* err;             // device error word (bounded waits of the tensor-core Gram)
     double* qws;          // global QR work space for bases too large for shared memory, or nullptr
+    // position VJP (vjp_entries): the field, the cotangents [noutputs][n], the
+    // per-entry gradients [nnz][dim] and each row's own sum of them [n][dim]
+    const double* f;
+    const double* gbar;
+    double* gentry;
+    double* gown;
 };
 
 // Scratch bytes per particle of an assembly batch (Gram entries,
@@ -409,21 +419,14 @@ cudaError_t vjp_field_sell(const VjpSellArgs& a, int nout, cudaStream_t s);
 cudaError_t transpose_outputs(const int64_t* tidx, int64_t nnz, int nout, const double* w64, const float* w32,
                               int64_t ws, double* wt, cudaStream_t s);
 
-struct VjpArgs {
-    const AsmTables* tab;
-    int64_t n;
-    const double* pos;
-    const int64_t* rowptr;
-    const int32_t* cols;
-    Geom geom;
-    double h_over_eps;
-    const double* eps_fixed;
-    const double* f;      // field [n]
-    const double* gbar;   // cotangent [noutputs][n]
-    double* gentry;       // scratch [nnz][dim]: dPhi_p / dx_pq
-};
-cudaError_t vjp_positions(const VjpArgs& a, const AsmTables& h, const int64_t* trow, const int64_t* tidx, double* grad,
-                          cudaStream_t s);
+// dPhi_p / dx_pq of every entry (a.gentry) and their sum over each row
+// (a.gown): eps, Gram, QR and chain-rule kernels over the assembly's batches
+// (a.eps and a.eip_group: scratch).  Scratch bytes per particle of a batch:
+int64_t vjp_scratch_bytes(const AsmTables& h, int maxk);
+cudaError_t vjp_entries(const AsmArgs& a, const AsmTables& h, cudaStream_t s);
+// grad[i] -= the entries' gradients of the transposed row i
+cudaError_t vjp_gather(const int64_t* trow, const int64_t* tidx, int64_t n, int dim, const double* gentry,
+                       double* grad, cudaStream_t s);
 
 // ------------------------------------------------- RK4 reaction-diffusion --
 template <typename T>
