@@ -5,7 +5,7 @@
 // particle by particle (src/Operators/Vector/cuda/vector_dist_operators_cuda.cuh
 // :444-461; the reference evaluates DC-PSE nodes on the host only).
 //
-//  * apply_term_f64: one reference Dcpse object, FP64, in the reference's
+//  * apply_terms_f64: reference Dcpse objects, FP64, in the reference's
 //    order  Df_p = (sum_q (f_q + s f_p) K_pq) * eps_p^-|alpha|.  Compiled with
 //    -fmad=false, so it matches the CPU oracle bit for bit.
 //  * batched applies: every output of a plan in one pass over the neighbour
@@ -32,6 +32,7 @@
 
 #include "dcpse_internal.h"
 #include "dcpse_f32_row.cuh"
+#include "dcpse_softfp.cuh"
 
 namespace dcpse {
 namespace {
@@ -63,70 +64,137 @@ __device__ __forceinline__ int64_t row_by_length(int64_t base, int64_t n, const 
     return p;         // >= n: no row for this thread
 }
 
-__global__ void __launch_bounds__(256) apply_term_f64_kernel(int64_t n, const int64_t* __restrict__ rowptr,
-                                                             const int32_t* __restrict__ cols,
-                                                             const double* __restrict__ K,
-                                                             const double* __restrict__ eip, double sign,
-                                                             const double* __restrict__ f, double* __restrict__ out,
-                                                             int accumulate) {
-    __shared__ int s_len[256], s_row[256];
-    for (int64_t base = (int64_t)blockIdx.x * 256; base < n; base += (int64_t)gridDim.x * 256) {
-        const int64_t p = row_by_length(base, n, rowptr, s_len, s_row);
-        if (p >= n) continue;
-        const double fxp = sign * f[p];
-        double D = 0.0;
-        const int64_t e = rowptr[p + 1];
-        int64_t j = rowptr[p];
-        // 4 entries in flight: all loads of a batch are issued first, the
-        // sum then takes them in row order
-        for (; j + 4 <= e; j += 4) {
-            int32_t q[4];
-            double k[4], fq[4];
+// T terms of one sign, each D_t = sum_q (f_q + s f_p) K_t,pq in row order,
+// then their outputs' sums in term order: one sum f_q + s f_p per entry serves
+// all terms, and the products run on the integer pipes, which leaves T + 1 FP64
+// operations per entry instead of 3 T.  FP64-pipe bound (82 % before its sums
+// became three-register dfmas); 96^3 Laplacian, three terms: 1.46 ms with a
+// launch per term and FP64 products, 0.78 ms fused with integer products,
+// 0.727 ms with the sums as dfmas.  Staging the rows through shared memory
+// (cp.async tiles, coalesced) was slower, 1.10 ms: its copies and the
+// occupancy it costs outweigh the line accesses it saves.
+struct TermsArgs {
+    int64_t n;
+    const int64_t* rowptr;
+    const int32_t* cols;
+    const double* K[kTermsFused];
+    const double* eip[kTermsFused];
+    double* out[kTermsFused];   // output of each term
+    unsigned fresh, last;       // bit t: term t begins / ends its output's terms in this launch
+    int accumulate;             // the first output continues an earlier launch
+    double sign;
+    const double* f;
+};
+
+// D[t] = D[t] + d[u] k[t][u] over the batch's first cnt entries u in order, with
+// the products on the integer pipes when every d (or its zero) and k of the
+// batch is in their range: one branch a batch, so that the products overlap
+template <int T, int U>
+__device__ __forceinline__ void add_products(const Fma& F, double (&D)[T], const double (&d)[U],
+                                             const double (&k)[T][U], int cnt) {
+    bool ok = true;
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                q[u] = cols[j + u];
-                k[u] = K[j + u];
+    for (int u = 0; u < U; ++u) {
+        ok = ok && int_range_or_zero(d[u]);
+#pragma unroll
+        for (int t = 0; t < T; ++t) ok = ok && int_range(k[t][u]);
+    }
+    if (ok) {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int t = 0; t < T; ++t) {
+                const double v = F.add(rn_mul_int(d[u], k[t][u]), D[t]);
+                D[t] = u < cnt ? v : D[t];
+            }
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int t = 0; t < T; ++t)
+                if (u < cnt) D[t] = D[t] + d[u] * k[t][u];
+    }
+}
+
+template <int T>
+__global__ void __launch_bounds__(256) apply_terms_f64_kernel(TermsArgs a) {
+    __shared__ int s_len[256], s_row[256];
+    const Fma F;
+    for (int64_t base = (int64_t)blockIdx.x * 256; base < a.n; base += (int64_t)gridDim.x * 256) {
+        const int64_t p = row_by_length(base, a.n, a.rowptr, s_len, s_row);
+        if (p >= a.n) continue;
+        const double fxp = a.sign * a.f[p];
+        double D[T];
+#pragma unroll
+        for (int t = 0; t < T; ++t) D[t] = 0.0;
+        const int64_t b = a.rowptr[p];
+        const int len = (int)(a.rowptr[p + 1] - b);
+        // U entries in flight: all loads of a batch are issued first, the
+        // sums then take them in row order
+        constexpr int U = 4;
+        for (int j = 0; j < len; j += U) {
+            int32_t q[U];
+            double k[T][U], fq[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const bool in = j + u < len;
+                q[u] = in ? a.cols[b + j + u] : (int32_t)p;
+#pragma unroll
+                for (int t = 0; t < T; ++t) k[t][u] = in ? a.K[t][b + j + u] : 1.0;
             }
 #pragma unroll
-            for (int u = 0; u < 4; ++u) fq[u] = f[q[u]];
+            for (int u = 0; u < U; ++u) fq[u] = a.f[q[u]];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) D = D + (fq[u] + fxp) * k[u];
+            for (int u = 0; u < U; ++u) fq[u] = F.add(fq[u], fxp);
+            add_products<T, U>(F, D, fq, k, len - j);
         }
-        for (; j < e; ++j) D = D + (f[cols[j]] + fxp) * K[j];
-        D = D * eip[p];
-        out[p] = accumulate ? out[p] + D : D;
+        double r = a.accumulate ? a.out[0][p] : 0.0;
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            const double v = D[t] * a.eip[t][p];
+            r = ((a.fresh >> t) & 1u) ? v : r + v;
+            if ((a.last >> t) & 1u) a.out[t][p] = r;
+        }
     }
 }
 
 // Dcpse::p2p (Dcpse.hpp:198-297): Df_p = epsInvPow_p * (sum_q f_q K_pq) per
 // component, f on the support set ([n_sup][ncomp]), out on the domain set.
-__global__ void __launch_bounds__(256) p2p_f64_kernel(int64_t n, const int64_t* __restrict__ rowptr,
+// Bound by the FP64 pipe and the L1's line accesses (a row per thread: 32
+// lines a load), so the products stay on the pipe, as dfmas: 64^3 periodic 128
+// us with dmul and dadd, 121 us; on the integer pipes they cost the occupancy
+// that hides the loads (146 us).
+__global__ void __launch_bounds__(256, 6) p2p_f64_kernel(int64_t n, const int64_t* __restrict__ rowptr,
                                                       const int32_t* __restrict__ cols, const double* __restrict__ K,
                                                       const double* __restrict__ eip, int ncomp,
                                                       const double* __restrict__ f, double* __restrict__ out) {
     __shared__ int s_len[256], s_row[256];
+    const Fma F;
     for (int64_t base = (int64_t)blockIdx.x * 256; base < n; base += (int64_t)gridDim.x * 256) {
         const int64_t p = row_by_length(base, n, rowptr, s_len, s_row);
         if (p >= n) continue;
-        const int64_t b = rowptr[p], e = rowptr[p + 1];
+        const int64_t b = rowptr[p];
+        const int len = (int)(rowptr[p + 1] - b);
+        const int32_t* __restrict__ cr = cols + b;
+        const double* __restrict__ Kr = K + b;
         for (int c = 0; c < ncomp; ++c) {
             double D = 0.0;
-            int64_t j = b;
+            int j = 0;
             // 4 entries in flight, summed in row order
-            for (; j + 4 <= e; j += 4) {
+            for (; j + 4 <= len; j += 4) {
                 int32_t q[4];
                 double k[4], fq[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    q[u] = cols[j + u];
-                    k[u] = K[j + u];
+                    q[u] = cr[j + u];
+                    k[u] = Kr[j + u];
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) fq[u] = f[(int64_t)q[u] * ncomp + c];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) D = D + fq[u] * k[u];
+                for (int u = 0; u < 4; ++u) D = F.add(F.mul(fq[u], k[u]), D);
             }
-            for (; j < e; ++j) D = D + f[(int64_t)cols[j] * ncomp + c] * K[j];
+            for (; j < len; ++j) D = F.add(F.mul(f[(int64_t)cr[j] * ncomp + c], Kr[j]), D);
             out[p * ncomp + c] = eip[p] * D;
         }
     }
@@ -573,14 +641,34 @@ cudaError_t launch_f64(int64_t n, int nout, const int64_t* rowptr, const int32_t
 
 }  // namespace
 
-cudaError_t apply_term_f64(int64_t n, const int64_t* rowptr, const int32_t* cols, const double* K, const double* eip,
-                           unsigned ord, const double* f, double* out, int accumulate, cudaStream_t s) {
-    if (n == 0) return cudaSuccess;
-    const double sign = (ord % 2 == 0) ? -1.0 : 1.0;
-    int64_t g = (n + 255) / 256;
-    int64_t cap = (int64_t)num_sms() * 8;
-    apply_term_f64_kernel<<<(unsigned)(g < cap ? g : cap), 256, 0, s>>>(n, rowptr, cols, K, eip, sign, f, out,
-                                                                         accumulate);
+// Terms of one output run (or several outputs), all of one sign, in plan order
+// (TermsArgs).  One launch for up to kTermsFused terms.
+cudaError_t apply_terms_f64(int64_t n, const int64_t* rowptr, const int32_t* cols, int nterms, const double* const* K,
+                            const double* const* eip, double* const* out, int accumulate, unsigned order,
+                            const double* f, cudaStream_t s) {
+    if (n == 0 || nterms == 0) return cudaSuccess;
+    if (nterms > kTermsFused) return cudaErrorInvalidValue;
+    TermsArgs a{};
+    a.n = n;
+    a.rowptr = rowptr;
+    a.cols = cols;
+    for (int t = 0; t < nterms; ++t) {
+        a.K[t] = K[t];
+        a.eip[t] = eip[t];
+        a.out[t] = out[t];
+        if (t == 0 ? !accumulate : out[t] != out[t - 1]) a.fresh |= 1u << t;
+        if (t + 1 == nterms || out[t + 1] != out[t]) a.last |= 1u << t;
+    }
+    a.accumulate = accumulate;
+    a.sign = (order % 2 == 0) ? -1.0 : 1.0;
+    a.f = f;
+    // a block per window: the block scheduler balances them
+    const unsigned grid = (unsigned)((n + 255) / 256);
+    switch (nterms) {
+        case 1: apply_terms_f64_kernel<1><<<grid, 256, 0, s>>>(a); break;
+        case 2: apply_terms_f64_kernel<2><<<grid, 256, 0, s>>>(a); break;
+        default: apply_terms_f64_kernel<3><<<grid, 256, 0, s>>>(a); break;
+    }
     return cudaGetLastError();
 }
 
@@ -595,9 +683,7 @@ cudaError_t split_f64(const double* f, int64_t n, float2* f2, cudaStream_t s, in
 cudaError_t p2p_f64(int64_t n, const int64_t* rowptr, const int32_t* cols, const double* K, const double* eip,
                     int ncomp, const double* f, double* out, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    int64_t g = (n + 255) / 256;
-    int64_t cap = (int64_t)num_sms() * 8;
-    p2p_f64_kernel<<<(unsigned)(g < cap ? g : cap), 256, 0, s>>>(n, rowptr, cols, K, eip, ncomp, f, out);
+    p2p_f64_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, rowptr, cols, K, eip, ncomp, f, out);
     return cudaGetLastError();
 }
 

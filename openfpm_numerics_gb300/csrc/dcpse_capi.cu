@@ -1921,20 +1921,43 @@ int dcpse_copy(void* dst, const void* src, uint64_t bytes) {
     return DCPSE_OK;
 }
 
+namespace {
+// The sum of `count` terms into d_out, in order: one launch per run of up to
+// kTermsFused terms of one sign.
+int apply_terms(dcpse_plan_t* P, const int* terms, int count, const double* d_f, double* d_out) {
+    auto order = [&](int t) {
+        unsigned o = 0;
+        for (int d = 0; d < P->dim; ++d) o += P->sigs[t][d];
+        return o;
+    };
+    for (int i = 0; i < count;) {
+        const double *K[kTermsFused], *eip[kTermsFused];
+        double* out[kTermsFused];
+        const unsigned ord = order(terms[i]);
+        int m = 0;
+        for (; m < kTermsFused && i + m < count && order(terms[i + m]) % 2 == ord % 2; ++m) {
+            const int t = terms[i + m];
+            K[m] = P->k_term + (size_t)t * P->nnz;
+            eip[m] = P->eip_group + (size_t)P->term_group[t] * P->n;
+            out[m] = d_out;
+        }
+        P->tstart(DCPSE_K_APPLY_TERM);
+        cudaError_t e = apply_terms_f64(P->n, P->rowptr, P->cols, m, K, eip, out, i > 0, ord, d_f, P->stream);
+        P->tstop(DCPSE_K_APPLY_TERM);
+        DCPSE_CK(e);
+        i += m;
+    }
+    return DCPSE_OK;
+}
+}  // namespace
+
 int dcpse_apply_term_f64(dcpse_plan_t* P, int term, const double* d_f, double* d_out) {
     if (int rc = check_plan(P)) return rc;
     if (int rc = check_single_set(P)) return rc;
     if (!P->assembled || !P->k_term) return fail(DCPSE_ERR_STATE, "per-term FP64 kernels not stored");
     if (term < 0 || term >= P->nterms) return fail(DCPSE_ERR_ARG, "term out of range");
     if (P->n > 0 && (!d_f || !d_out)) return fail(DCPSE_ERR_ARG, "NULL field");
-    unsigned ord = 0;
-    for (int d = 0; d < P->dim; ++d) ord += P->sigs[term][d];
-    P->tstart(DCPSE_K_APPLY_TERM);
-    cudaError_t e = apply_term_f64(P->n, P->rowptr, P->cols, P->k_term + (size_t)term * P->nnz,
-                                   P->eip_group + (size_t)P->term_group[term] * P->n, ord, d_f, d_out, 0, P->stream);
-    P->tstop(DCPSE_K_APPLY_TERM);
-    DCPSE_CK(e);
-    return DCPSE_OK;
+    return apply_terms(P, &term, 1, d_f, d_out);
 }
 
 int dcpse_apply_output_f64(dcpse_plan_t* P, int output, const double* d_f, double* d_out) {
@@ -1943,20 +1966,10 @@ int dcpse_apply_output_f64(dcpse_plan_t* P, int output, const double* d_f, doubl
     if (!P->assembled || !P->k_term) return fail(DCPSE_ERR_STATE, "per-term FP64 kernels not stored");
     if (output < 0 || output >= P->nout) return fail(DCPSE_ERR_ARG, "output out of range");
     if (P->n > 0 && (!d_f || !d_out)) return fail(DCPSE_ERR_ARG, "NULL field");
-    int first = 1;
-    for (int t = 0; t < P->nterms; ++t) {
-        if (P->term_output[t] != output) continue;
-        unsigned ord = 0;
-        for (int d = 0; d < P->dim; ++d) ord += P->sigs[t][d];
-        P->tstart(DCPSE_K_APPLY_TERM);
-        cudaError_t e = apply_term_f64(P->n, P->rowptr, P->cols, P->k_term + (size_t)t * P->nnz,
-                                       P->eip_group + (size_t)P->term_group[t] * P->n, ord, d_f, d_out,
-                                       first ? 0 : 1, P->stream);
-        P->tstop(DCPSE_K_APPLY_TERM);
-        DCPSE_CK(e);
-        first = 0;
-    }
-    return DCPSE_OK;
+    std::vector<int> terms;
+    for (int t = 0; t < P->nterms; ++t)
+        if (P->term_output[t] == output) terms.push_back(t);
+    return apply_terms(P, terms.data(), (int)terms.size(), d_f, d_out);
 }
 
 namespace {

@@ -1,0 +1,46 @@
+// rn_mul_int against the host's IEEE product, bit for bit: random significands,
+// short ones (ties), all-ones ones, every exponent of its range, signed zeros.
+#include <cstdio>
+#include <cstdint>
+#include <cstring>
+
+#include "dcpse_softfp.cuh"
+
+using namespace dcpse;
+
+static uint64_t st = 0x9E3779B97F4A7C15ull;
+static uint64_t rnd() {
+    st ^= st << 13;
+    st ^= st >> 7;
+    st ^= st << 17;
+    return st;
+}
+
+static double draw(int kind) {
+    uint64_t m = rnd() & 0xfffffffffffffull;
+    if (kind & 1) m &= ~((1ull << (rnd() % 53)) - 1);
+    if (kind & 2) m |= 0xfffffffff0000ull;
+    if (kind & 4) m = (rnd() & 1) ? 0 : 0xfffffffffffffull - (rnd() & 3);
+    const uint64_t e = (kind & 8) ? ((rnd() & 1) ? 768 : 1279) : 768 + rnd() % 512;
+    const uint64_t u = (rnd() & (1ull << 63)) | (e << 52) | m;
+    double d;
+    std::memcpy(&d, &u, 8);
+    return (kind == 15 && (rnd() & 1)) ? 0.0 * d : d;
+}
+
+int main() {
+    for (long i = 0; i < 20000000; ++i) {
+        const double a = draw((int)(i & 15)), b = draw((int)((i >> 4) & 15));
+        if (!int_range_or_zero(a) || !int_range_or_zero(b)) return 2;
+        volatile double h = a * b;
+        const double r = rn_mul_int(a, b);
+        if (dbits(h) != dbits(r)) {
+            std::printf("%a * %a = %a, not %a\n", a, b, (double)h, r);
+            return 1;
+        }
+    }
+    const double out[] = {0x1p-256, 0x1p257, 5e-324, 1.0 / 0.0, 0.0 / 0.0};
+    for (double x : out)
+        if (int_range_or_zero(x) || int_range_or_zero(-x)) return 3;
+    return 0;
+}
