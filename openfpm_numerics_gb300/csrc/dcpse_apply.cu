@@ -70,7 +70,8 @@ __device__ __forceinline__ int64_t row_by_length(int64_t base, int64_t n, const 
 // operations per entry instead of 3 T.  FP64-pipe bound (82 % before its sums
 // became three-register dfmas); 96^3 Laplacian, three terms: 1.46 ms with a
 // launch per term and FP64 products, 0.78 ms fused with integer products,
-// 0.727 ms with the sums as dfmas.  Staging the rows through shared memory
+// 0.646 ms with the sums as dfmas and no comparison left on the pipe (L1 line
+// accesses 88 %, FP64 79 %).  Staging the rows through shared memory
 // (cp.async tiles, coalesced) was slower, 1.10 ms: its copies and the
 // occupancy it costs outweigh the line accesses it saves.
 struct TermsArgs {

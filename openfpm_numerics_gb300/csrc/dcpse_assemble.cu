@@ -39,7 +39,10 @@
 
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "dcpse_internal.h"
+#include "dcpse_softfp.cuh"
 
 namespace dcpse {
 namespace {
@@ -55,6 +58,7 @@ struct Split {
     int nrhs[kMaxGroups];    // right-hand sides per group (per term or per output)
     int c_off[kMaxGroups];   // coefficient block of each group, [gn][nrhs]
     int nmax;                // largest basis
+    int nrmax;               // most right-hand sides of a group
     int qwords;              // doubles of the largest [A|b] plus its solution block
     int pstride;             // doubles of QR work space per particle (set per lane grouping)
     int ldb;                 // row stride of the B chunk of the Gram kernel
@@ -84,6 +88,8 @@ __device__ __forceinline__ void load_offset(const AsmArgs& a, const double* xp, 
     for (int d = 0; d < DIM; ++d) o[d] = offset1(a.geom, d, xp[d], a.spos[q * DIM + d]);
 }
 
+// bit of a status word: the coefficients of group g are in coef_range_or_zero
+__device__ __forceinline__ int coef_bit(int g) { return 1 << (16 + g); }
 __device__ __forceinline__ int group_status(int32_t word, int g) { return (word >> (4 * g)) & 15; }
 
 // isfinite on the exponent bits (integer pipe, not the FP64 one)
@@ -115,6 +121,17 @@ __device__ __forceinline__ void monomials(const double* u, double* V, const Prog
     V[DIM * 32 + lane] = 1.0;
     for (int o = 0; o < nprog; ++o)
         V[(DIM + 1 + o) * 32 + lane] = V[P.prog[o][0] * 32 + lane] * V[P.prog[o][1] * 32 + lane];
+}
+
+// The same on the integer pipes, for u in unit_range_or_zero (every power and
+// product of the program is then in the range, or a zero).
+template <int DIM>
+__device__ __forceinline__ void monomials_int(const double* u, double* V, const ProgShared& P, int nprog, int lane) {
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) V[d * 32 + lane] = u[d];
+    V[DIM * 32 + lane] = 1.0;
+    for (int o = 0; o < nprog; ++o)
+        V[(DIM + 1 + o) * 32 + lane] = rn_mul_int(V[P.prog[o][0] * 32 + lane], V[P.prog[o][1] * 32 + lane]);
 }
 
 // ----------------------------------------------------------------- 0. eps --
@@ -510,15 +527,20 @@ __global__ void __launch_bounds__(kQrWarps * 32) qr_kernel(AsmArgs a, Split S, i
                 }
             }
             __syncwarp();
+            bool in_range = true;
             if (!dead) {
                 double* C = S.coef + slot * S.cstride + S.c_off[g];
                 for (int e = l; e < n * nrhs; e += LPP) {
                     const int i = e / nrhs, r = e - i * nrhs;
-                    C[perm[i] * nrhs + r] = Z[i * nrhs + r];
+                    const double z = Z[i * nrhs + r];
+                    C[perm[i] * nrhs + r] = z;
+                    in_range = in_range && coef_range_or_zero(z);
                 }
             } else if (active) {
                 word = (word & ~(15 << (4 * g))) | (ST_SINGULAR << (4 * g));
             }
+            const unsigned lanes = LPP == 32 ? 0xffffffffu : ((1u << LPP) - 1u) << (sub * LPP);
+            if ((__ballot_sync(0xffffffffu, in_range) & lanes) == lanes) word |= coef_bit(g);
             __syncwarp();
         }
         if (valid && l == 0) S.gst[slot] = word;
@@ -526,21 +548,69 @@ __global__ void __launch_bounds__(kQrWarps * 32) qr_kernel(AsmArgs a, Split S, i
 }
 
 // ------------------------------------------------------------- 3. weights --
-// One warp per particle, one neighbour row per lane.  The right-hand sides
-// and outputs are run-time loops (no work predicated off on the FP64 pipe);
-// per-output sums live in this lane's column of shared memory.
+// NR right-hand sides of one group and one neighbour row in the reference's
+// order, res_r = sum_i (A_ir V_i) ef (coefficients A of row stride ld).  INT: the
+// products on the integer pipes, but every other product with ef, which keeps
+// both pipes about equally busy (uneven 2D cloud, five terms: 1.47 ms with all
+// of them on the integer pipes, at 66 % of those and 56 % of the FP64 pipe).
+template <int NR, bool INT>
+__device__ __forceinline__ void reference_sums(const Fma& F, const double* __restrict__ A, int ld, int n,
+                                               const unsigned char* gslot, const double* V, int lane, double ef,
+                                               double (&res)[NR]) {
+#pragma unroll 2
+    for (int i = 0; i < n; ++i) {
+        const double v = V[gslot[i] * 32 + lane];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            const double t = INT ? rn_mul_int(A[i * ld + r], v) : F.mul(A[i * ld + r], v);
+            res[r] = F.add(INT && (i & 1) == 0 ? rn_mul_int(t, ef) : F.mul(t, ef), res[r]);
+        }
+    }
+}
+
+// res_r = sum_i A_ir V_i by fused multiply-adds (fast assembly)
+template <int NR>
+__device__ __forceinline__ void fast_sums(const double* __restrict__ A, int ld, int n, const unsigned char* gslot,
+                                          const double* V, int lane, double (&res)[NR]) {
+    for (int i = 0; i < n; ++i) {
+        const double v = V[gslot[i] * 32 + lane];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) res[r] = fma(A[i * ld + r], v, res[r]);
+    }
+}
+
+// The entries of up to 32 consecutive particles, one per lane: a warp takes
+// `per_warp` particles, concatenates their rows and walks them 32 entries at a
+// time (a binary search over the rows' ends gives a lane its particle), so that
+// only the last step of all has idle lanes.  The particles' coefficients are
+// read through L1; per-output sums live in this lane's column of shared memory.
+//
+// FP64-pipe bound: a warp per particle with its rows in chunks of 32 ran 14 %
+// (3D) to 40 % (uneven 2D clouds) of its lanes idle, and in the reference's
+// order every coefficient took two products and a sum on the pipe.  Now the
+// monomials, the reference order's products and the scalings are on the integer
+// pipes, the sums are three-register dfmas and the FP32 narrowing is on integers:
+// 2e5 uneven particles, five terms in the reference's order 3.18 -> 1.34 ms; 80^3
+// Gradient + Laplacian, fast assembly, a batch of 1.2e5 particles 2.44 -> 1.59 ms.
 template <int DIM>
-__global__ void __launch_bounds__(256) weights_kernel(AsmArgs a, Split S, int64_t b0, int64_t b1) {
+__global__ void __launch_bounds__(256) weights_kernel(AsmArgs a, Split S, int64_t b0, int64_t b1, int per_warp) {
     extern __shared__ double smem[];
     __shared__ ProgShared P;
+    __shared__ ExpShared X;
+    __shared__ unsigned char gslot[kMaxGroups][kMaxBasis];  // slot of basis function i of group g
     const AsmTables& T = *a.tab;
-    stage_program(T, P);
+    const int ngroups = T.ngroups;
+    for (int g = 0; g < ngroups; ++g)
+        for (int i = threadIdx.x; i < T.gn[g]; i += blockDim.x) gslot[g][i] = T.uslot[T.gidx[g][i]];
+    stage_exp(X);
+    stage_program(T, P);  // (ends with a barrier)
+    const Fma F;
+    const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    double* Cs = smem + (size_t)wib * (S.cstride + (S.nslots + S.nout) * 32);
-    double* V = Cs + S.cstride;
+    double* V = smem + (size_t)wib * (S.nslots + S.nout + S.nrmax) * 32;
     double* Wacc = V + S.nslots * 32;
-    const int ngroups = T.ngroups;
+    double* R = Wacc + S.nout * 32;
     const int nprog = T.nprog;
     const bool fast = (a.flags & DCPSE_ASSEMBLE_FAST_FLAG) != 0;
     const bool st_terms = a.k_term != nullptr;
@@ -548,85 +618,153 @@ __global__ void __launch_bounds__(256) weights_kernel(AsmArgs a, Split S, int64_
 
     const int wpc = blockDim.x >> 5;
     const int64_t nw = (int64_t)gridDim.x * wpc;
-    for (int64_t it = b0 + (int64_t)blockIdx.x * wpc + wib; it < b1; it += nw) {
-        const int64_t slot = it - b0;
-        const int64_t p = a.order ? (int64_t)a.order[it] : it;
-        const int64_t beg = a.rowptr[p];
-        const int k = (int)(a.rowptr[p + 1] - beg);
-        const double eps = a.eps[p];
-        const int32_t word = S.gst[slot];
-        for (int e = lane; e < S.cstride; e += 32) Cs[e] = S.coef[slot * S.cstride + e];
-        __syncwarp();
-
-        double eipg[kMaxGroups];
+    for (int64_t t0 = b0 + ((int64_t)blockIdx.x * wpc + wib) * per_warp; t0 < b1; t0 += nw * per_warp) {
+        // lane l holds particle t0 + l of the warp's group
+        const int np = (int)min((int64_t)per_warp, b1 - t0);
+        int64_t lp = 0, lbeg = 0;
+        int32_t lword = 0;
+        int lk = 0;
+        if (lane < np) {
+            lp = a.order ? (int64_t)a.order[t0 + lane] : t0 + lane;
+            lbeg = a.rowptr[lp];
+            lk = (int)(a.rowptr[lp + 1] - lbeg);
+            lword = S.gst[t0 + lane - b0];
+        }
+        int lend = lk;  // inclusive scan of the row lengths
 #pragma unroll
-        for (int g = 0; g < kMaxGroups; ++g) eipg[g] = (g < ngroups) ? 1.0 / ipow(eps, (unsigned)T.gord[g]) : 0.0;
-        bool nonfinite = false;
-        for (int c0 = 0; c0 < k; c0 += kCh) {
-            int q = c0 + lane;
-            if (q >= k) break;  // rows of this lane are done; no warp sync below
-            // u = x_pq / eps as the Gram kernel computed it (rows of particles
-            // with no assembled group were skipped there and are not used here)
-            double u[DIM];
-            const double* Ur = S.usc + slot * S.ustride;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(full, lend, o);
+            if (lane >= o) lend += v;
+        }
+        const int total = __shfl_sync(full, lend, 31);
+        unsigned bad = 0;  // particles of the group with a non-finite kernel
+        for (int e0 = 0; e0 < total; e0 += 32) {
+            const int e = e0 + lane;
+            int s = 0, hi = np - 1;  // first particle whose rows end past e
 #pragma unroll
-            for (int d = 0; d < DIM; ++d) u[d] = Ur[d * S.maxk + q];
-            monomials<DIM>(u, V, P, nprog, lane);
-            const double ef = cw_exp(-norm2<DIM>(u));
-            for (int t = 0; t < noutputs; ++t) Wacc[t * 32 + lane] = 0.0;
-            for (int g = 0; g < ngroups; ++g) {
-                const int n = T.gn[g];
-                const int nrhs = S.nrhs[g];
-                const bool ok = group_status(word, g) == ST_OK;
-                const double* Ag = Cs + S.c_off[g];
-                double eip = eipg[0];
-#pragma unroll
-                for (int t = 1; t < kMaxGroups; ++t)
-                    if (t == g) eip = eipg[t];
-                for (int r = 0; r < nrhs; ++r) {
-                    double res = 0.0;
-                    if (ok) {
-                        if (fast) {
-                            for (int i = 0; i < n; ++i)
-                                res = fma(Ag[i * nrhs + r], V[P.uslot[T.gidx[g][i]] * 32 + lane], res);
-                        } else {
-                            for (int i = 0; i < n; ++i) {
-                                double t0 = Ag[i * nrhs + r] * V[P.uslot[T.gidx[g][i]] * 32 + lane];
-                                t0 = t0 * ef;
-                                res = res + t0;
-                            }
-                        }
-                    }
-                    double Kq;
-                    int o2;
-                    if (fast) {
-                        Kq = ok ? (res * ef) : 0.0;
-                        o2 = T.out_of_rhs[g][r];
-                    } else {
-                        Kq = res;
-                        const int term = T.term_of_rhs[g][r];
-                        if (st_terms) a.k_term[(int64_t)term * a.nnz + beg + q] = Kq;
-                        o2 = T.term_output[term];
-                    }
-                    nonfinite |= !finite_bits(Kq);
-                    Wacc[o2 * 32 + lane] = Wacc[o2 * 32 + lane] + Kq * eip;
+            for (int it = 0; it < 5; ++it) {
+                const int mid = (s + hi) >> 1;
+                const int v = __shfl_sync(full, lend, mid);
+                if (s < hi) {
+                    if (v > e)
+                        hi = mid;
+                    else
+                        s = mid + 1;
                 }
             }
-            for (int t = 0; t < noutputs; ++t) {
-                const double w = Wacc[t * 32 + lane];
-                if (a.w64) a.w64[(int64_t)t * a.nnz + beg + q] = w;
-                const float w32 = (float)w;
-                if (a.w32) a.w32[(int64_t)t * a.nnz + beg + q] = w32;
-                if (a.r16)
-                    reinterpret_cast<__nv_bfloat16*>(a.r16)[(int64_t)t * a.nnz + beg + q] =
-                        __float2bfloat16_rn((float)(w - (double)w32));
-                if (a.r32) a.r32[(int64_t)t * a.nnz + beg + q] = (float)(w - (double)w32);
+            const int q = e - (__shfl_sync(full, lend, s) - __shfl_sync(full, lk, s));
+            const int64_t at = __shfl_sync(full, lbeg, s) + q;
+            const int64_t p = __shfl_sync(full, lp, s);
+            const int32_t word = __shfl_sync(full, lword, s);
+            bool nonfinite = false;
+            if (e < total) {
+                const int64_t slot = t0 - b0 + s;
+                // u = x_pq / eps as the Gram kernel computed it (rows of particles
+                // with no assembled group were skipped there and are not used here)
+                double u[DIM];
+                const double* Ur = S.usc + slot * S.ustride + q;
+                bool unit = true;
+#pragma unroll
+                for (int d = 0; d < DIM; ++d) {
+                    u[d] = Ur[d * S.maxk];
+                    unit = unit && unit_range_or_zero(u[d]);
+                }
+                double u2;
+                if (unit) {
+                    monomials_int<DIM>(u, V, P, nprog, lane);
+                    u2 = rn_mul_int(u[0], u[0]);
+#pragma unroll
+                    for (int d = 1; d < DIM; ++d) u2 = F.add(rn_mul_int(u[d], u[d]), u2);
+                } else {
+                    monomials<DIM>(u, V, P, nprog, lane);
+                    u2 = norm2<DIM>(u);
+                }
+                const double ef = cw_exp(F, X, -u2);
+                const bool ints = unit && int_range(ef);
+                for (int t = 0; t < noutputs; ++t) Wacc[t * 32 + lane] = 0.0;
+                for (int g = 0; g < ngroups; ++g) {
+                    const int n = T.gn[g];
+                    const int nrhs = S.nrhs[g];
+                    const bool ok = group_status(word, g) == ST_OK;
+                    const double* __restrict__ Ag = S.coef + slot * S.cstride + S.c_off[g];
+                    const double eip = a.eip_group[(int64_t)g * a.n + p];
+                    // the sums of NR right-hand sides from r0 on, to this lane's
+                    // column of R
+                    auto block = [&](int r0, auto count) {
+                        constexpr int NR = decltype(count)::value;
+                        double res[NR];
+#pragma unroll
+                        for (int r = 0; r < NR; ++r) res[r] = 0.0;
+                        if (fast)
+                            fast_sums<NR>(Ag + r0, nrhs, n, gslot[g], V, lane, res);
+                        else
+                            reference_sums<NR, true>(F, Ag + r0, nrhs, n, gslot[g], V, lane, ef, res);
+#pragma unroll
+                        for (int r = 0; r < NR; ++r) R[(r0 + r) * 32 + lane] = res[r];
+                    };
+                    if (!ok) {
+                        for (int r = 0; r < nrhs; ++r) R[r * 32 + lane] = 0.0;
+                    } else if (!fast && !(ints && (word & coef_bit(g)))) {
+                        for (int r = 0; r < nrhs; ++r) {
+                            double res[1] = {0.0};
+                            reference_sums<1, false>(F, Ag + r, nrhs, n, gslot[g], V, lane, ef, res);
+                            R[r * 32 + lane] = res[0];
+                        }
+                    } else {
+                        int r0 = 0;
+                        for (; r0 + 3 <= nrhs; r0 += 3) block(r0, std::integral_constant<int, 3>{});
+                        if (nrhs - r0 == 2)
+                            block(r0, std::integral_constant<int, 2>{});
+                        else if (nrhs - r0 == 1)
+                            block(r0, std::integral_constant<int, 1>{});
+                    }
+#pragma unroll 1
+                    for (int r = 0; r < nrhs; ++r) {
+                        const double res = R[r * 32 + lane];
+                        const double Kq = fast && ok ? F.prod(res, ef) : res;
+                        int o2;
+                        if (fast) {
+                            o2 = T.out_of_rhs[g][r];
+                        } else {
+                            const int term = T.term_of_rhs[g][r];
+                            if (st_terms) a.k_term[(int64_t)term * a.nnz + at] = Kq;
+                            o2 = T.term_output[term];
+                        }
+                        nonfinite |= !finite_bits(Kq);
+                        const double w = Wacc[o2 * 32 + lane], v = F.prod(Kq, eip);
+                        // (0.0 + v is v but for v = -0.0)
+                        double sum;
+                        if (is_plus_zero(w))
+                            sum = is_zero(v) ? 0.0 : v;
+                        else
+                            sum = pipe_fma(v, F.one, w);
+                        Wacc[o2 * 32 + lane] = sum;
+                    }
+                }
+#pragma unroll 1
+                for (int t = 0; t < noutputs; ++t) {
+                    const double w = Wacc[t * 32 + lane];
+                    const int64_t i = (int64_t)t * a.nnz + at;
+                    if (a.w64) a.w64[i] = w;
+                    if (a.w32) {
+                        const float w32 = narrow(w);
+                        a.w32[i] = w32;
+                        if (a.r16 || a.r32) {
+                            const float r = narrow(F.add(w, -widen(w32)));
+                            if (a.r16) reinterpret_cast<__nv_bfloat16*>(a.r16)[i] = __float2bfloat16_rn(r);
+                            if (a.r32) a.r32[i] = r;
+                        }
+                    }
+                }
             }
+            bad |= __reduce_or_sync(full, nonfinite ? 1u << s : 0u);
         }
-        nonfinite = __any_sync(0xffffffffu, nonfinite);
-        if (nonfinite) {
+        for (unsigned m = bad; m; m &= m - 1) {
             // zero every stored row of this particle (the oracle zeroes the
             // affected term's kernels; fused outputs are zeroed entirely)
+            const int s = __ffs(m) - 1;
+            const int64_t beg = __shfl_sync(full, lbeg, s);
+            const int k = __shfl_sync(full, lk, s);
             for (int q = lane; q < k; q += 32) {
                 if (st_terms)
                     for (int t = 0; t < T.nterms; ++t) a.k_term[(int64_t)t * a.nnz + beg + q] = 0.0;
@@ -639,12 +777,12 @@ __global__ void __launch_bounds__(256) weights_kernel(AsmArgs a, Split S, int64_
                 }
             }
         }
-        if (lane == 0) {
+        if (lane < np) {
             int st = ST_OK;
             for (int g = 0; g < ngroups; ++g)
-                if (st == ST_OK && group_status(word, g) != ST_OK) st = group_status(word, g);
-            if (st == ST_OK && nonfinite) st = ST_NONFINITE;
-            a.status[p] = st;
+                if (st == ST_OK && group_status(lword, g) != ST_OK) st = group_status(lword, g);
+            if (st == ST_OK && ((bad >> lane) & 1u)) st = ST_NONFINITE;
+            a.status[lp] = st;
         }
         __syncwarp();
     }
@@ -744,15 +882,20 @@ cudaError_t launch_qr(const AsmArgs& a, Split S, int64_t b0, int64_t nb, cudaStr
 template <int DIM>
 cudaError_t launch_weights(const AsmArgs& a, const Split& S, int64_t b0, int64_t b1, cudaStream_t s) {
     int warps = warps_of(a);
-    const size_t per_warp = (size_t)(S.cstride + (S.nslots + S.nout) * 32) * sizeof(double);
-    // large bases: as many warps as their coefficients and monomials leave room for
+    const size_t per_warp = (size_t)((S.nslots + S.nout + S.nrmax) * 32) * sizeof(double);
+    // large bases: as many warps as their monomials leave room for
     warps = std::max(1, std::min(warps, smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024) / (int)per_warp));
     const size_t bytes = per_warp * warps;
     auto kern = weights_kernel<DIM>;
+    // particles a warp takes at a time: 16 leave a few idle lanes in a hundred,
+    // fewer when that would leave warps of the GPU without any
+    const int64_t nb = b1 - b0;
+    const int64_t chip = (int64_t)num_sms() * 32;
+    const int take = (int)std::max<int64_t>(1, std::min<int64_t>(16, nb / chip));
     int grid = 0;
-    cudaError_t e = persistent(kern, warps * 32, bytes, warps, b1 - b0, grid);
+    cudaError_t e = persistent(kern, warps * 32, bytes, (int64_t)warps * take, nb, grid);
     if (e != cudaSuccess) return e;
-    kern<<<grid, warps * 32, bytes, s>>>(a, S, b0, b1);
+    kern<<<grid, warps * 32, bytes, s>>>(a, S, b0, b1, take);
     return cudaGetLastError();
 }
 
@@ -877,6 +1020,7 @@ Split make_split(const AsmTables& h, int flags, bool vjp = false) {
         S.c_off[g] = off;
         off += n * S.nrhs[g];
         S.nmax = std::max(S.nmax, n);
+        S.nrmax = std::max(S.nrmax, S.nrhs[g]);
         S.qwords = std::max(S.qwords, n * (n + S.nrhs[g]) + n * S.nrhs[g]);
     }
     S.cstride = (off + 1) & ~1;

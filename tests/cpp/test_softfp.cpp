@@ -34,7 +34,7 @@ int main() {
         if (!int_range_or_zero(a) || !int_range_or_zero(b)) return 2;
         volatile double h = a * b;
         const double r = rn_mul_int(a, b);
-        if (dbits(h) != dbits(r)) {
+        if (dhi(h) != dhi(r) || dlo(h) != dlo(r)) {
             std::printf("%a * %a = %a, not %a\n", a, b, (double)h, r);
             return 1;
         }
