@@ -108,6 +108,32 @@ DCPSE_HD double rn_mul_int(double a, double b) {
     return from_bits(zero ? sign : ((uint32_t)(r >> 32) | sign), zero ? 0u : (uint32_t)r);
 }
 
+// RN(a / b) for a (or its zero), b and r in int_range, r within an ulp or two of
+// 1 / b: the quotient a r is off by a few ulps at most, and its exact remainder
+// A 2^s - B Q (significands as integers; it fits 64 bits, so only its low 64 are
+// formed) says which neighbour is nearest (the final-rounding argument of Markstein,
+// IBM J. Res. Dev. 34, 1990, in integers; a quotient is never half way).  False,
+// for the caller to divide, where the quotient is a power of two from above
+// (the spacing changes there) or more than one ulp off.
+DCPSE_HD bool rn_div_int(double a, double b, double r, double& q) {
+    q = rn_mul_int(a, r);
+    if (is_zero(q)) return true;
+    const uint32_t ah = dhi(a), bh = dhi(b), qh = dhi(q), ql = dlo(q), bl = dlo(b);
+    const uint32_t bm = (bh & 0xfffffu) | 0x100000u, qm = (qh & 0xfffffu) | 0x100000u;
+    // exponent of q below that of A / B in [1/2, 2): 0 or 1 (or -1 for a quotient rounded up to 2)
+    const int down = (int)((ah >> 20) & 0x7ffu) - (int)((bh >> 20) & 0x7ffu) + 1023 - (int)((qh >> 20) & 0x7ffu);
+    const uint64_t num = (uint64_t)(dlo(a) << (20 + down)) << 32;
+    int64_t rem = (int64_t)(num - ((uint64_t)bl * ql + ((uint64_t)(bl * qm + bm * ql) << 32)));
+    const int64_t B = (int64_t)(((uint64_t)bm << 32) | bl);
+    const bool low = qm == 0x100000u && ql == 0u && rem < 0;
+    const int up = 2 * rem > B, dn = 2 * rem < -B;
+    rem -= up ? B : 0;
+    rem += dn ? B : 0;
+    const uint64_t bits = ((((uint64_t)qh << 32) | ql) + (uint64_t)(int64_t)(up - dn));
+    q = from_bits((uint32_t)(bits >> 32), (uint32_t)bits);
+    return 2 * rem <= B && 2 * rem >= -B && !low && !((bits & 0xfffffffffffffull) == 0 && rem < 0);
+}
+
 // Whether x is 0 or 2^-16 <= |x| < 2^17: products of up to 8 such factors stay
 // within 2^136, and the product of one of those and a number below 2^101 (or a
 // zero) in int_range
@@ -172,6 +198,12 @@ struct Fma {
         : one(*(const volatile double*)&g_fma_one), nzero(*(const volatile double*)&g_fma_nzero) {}
     __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
     __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, nzero); }
+    // a / b, r = 1 / b to an ulp (the same r serves every dividend)
+    __device__ __forceinline__ double quot(double a, double b, double r) const {
+        double q;
+        if (int_range_or_zero(a) && int_range(b) && int_range(r) && rn_div_int(a, b, r, q)) return q;
+        return a / b;
+    }
     // a b on the integer pipes where both are in their range
     __device__ __forceinline__ double prod(double a, double b) const {
         if (int_range_or_zero(a) && int_range_or_zero(b)) return rn_mul_int(a, b);

@@ -1,5 +1,6 @@
-// rn_mul_int against the host's IEEE product, bit for bit: random significands,
-// short ones (ties), all-ones ones, every exponent of its range, signed zeros.
+// rn_mul_int and rn_div_int against the host's IEEE product and quotient, bit for
+// bit: random significands, short ones (ties), all-ones ones, every exponent of
+// their range, signed zeros; the quotient with reciprocals off by up to two ulps.
 #include <cstdio>
 #include <cstdint>
 #include <cstring>
@@ -39,6 +40,24 @@ int main() {
             return 1;
         }
     }
+    long divided = 0;
+    for (long i = 0; i < 20000000; ++i) {
+        const double a = draw((int)(i & 15)), b = draw((int)((i >> 4) & 7));
+        volatile double vr = 1.0 / b, h = a / b;
+        double r = vr, q;
+        const uint64_t u = (((uint64_t)dhi(r) << 32) | dlo(r)) + (uint64_t)((i >> 8) % 5) - 2;
+        std::memcpy(&r, &u, 8);
+        if (!int_range(r) || !rn_div_int(a, b, r, q)) {
+            ++divided;
+            continue;
+        }
+        if (dhi(h) != dhi(q) || dlo(h) != dlo(q)) {
+            std::printf("%a / %a = %a, not %a\n", a, b, (double)h, q);
+            return 4;
+        }
+    }
+    std::printf("left to the caller: %ld\n", divided);
+    if (divided > 10000000) return 5;
     const double out[] = {0x1p-256, 0x1p257, 5e-324, 1.0 / 0.0, 0.0 / 0.0};
     for (double x : out)
         if (int_range_or_zero(x) || int_range_or_zero(-x)) return 3;
