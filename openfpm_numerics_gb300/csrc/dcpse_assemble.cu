@@ -59,6 +59,7 @@ struct Split {
     int c_off[kMaxGroups];   // coefficient block of each group, [gn][nrhs]
     int nmax;                // largest basis
     int nrmax;               // most right-hand sides of a group
+    int qtab;                // Gram entries (i <= j) of all groups
     int qwords;              // doubles of the largest [A|b] plus its solution block
     int pstride;             // doubles of QR work space per particle (set per lane grouping)
     int ldb;                 // row stride of the B chunk of the Gram kernel
@@ -452,7 +453,7 @@ __global__ void __launch_bounds__(256) gram_b_kernel(AsmArgs a, Split S, int64_t
 // barrier is reached by the whole warp.  A group whose factorisation breaks
 // down (or that was not assembled) keeps running on its own work space and
 // only its stores are suppressed.
-template <int LPP>
+template <int LPP, bool WS>
 __global__ void __launch_bounds__(kQrWarps * 32) qr_kernel(AsmArgs a, Split S, int64_t b0, int64_t nb) {
     constexpr int PPW = 32 / LPP;
     extern __shared__ double smem[];
@@ -465,18 +466,38 @@ __global__ void __launch_bounds__(kQrWarps * 32) qr_kernel(AsmArgs a, Split S, i
     const int wpc = blockDim.x >> 5;
     const int pidx = wib * PPW + sub;  // particle slot of this lane group in the CTA
     // work space: shared memory, or a global slot per lane group when the
-    // basis is too large for it (S.qws)
+    // basis is too large for it (WS); a template argument, so that the shared
+    // one is addressed as such
     const int64_t gslot = ((int64_t)blockIdx.x * wpc + wib) * PPW + sub;
-    double* R = S.qws ? S.qws + gslot * S.pstride : smem + (size_t)pidx * S.pstride;
-    int* perm = S.qws ? S.qperm + gslot * S.nmax
-                      : reinterpret_cast<int*>(smem + (size_t)wpc * PPW * S.pstride) + pidx * S.nmax;
+    double* R = WS ? S.qws + gslot * S.pstride : smem + (size_t)pidx * S.pstride;
+    int* perm = WS ? S.qperm + gslot * S.nmax
+                   : reinterpret_cast<int*>(smem + (size_t)wpc * PPW * S.pstride) + pidx * S.nmax;
+    // the Gram entry of every (i <= j) of every group, as entry << 16 | i << 8 | j
+    uint32_t* tab = reinterpret_cast<uint32_t*>(smem + (size_t)wpc * PPW * S.pstride) + wpc * PPW * S.nmax;
+    if (!WS && S.qtab) {
+        int base = 0;
+        for (int g = 0; g < T.ngroups; ++g) {
+            const int n = T.gn[g];
+            for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+                const int i = e / n, j = e - i * n;
+                if (i > j) continue;
+                const int ui = T.gidx[g][i], uj = T.gidx[g][j];
+                tab[base + j * (j + 1) / 2 + i] =
+                    (uint32_t)T.upair[min(ui, uj)][max(ui, uj)] << 16 | (uint32_t)i << 8 | (uint32_t)j;
+            }
+            base += n * (n + 1) / 2;
+        }
+        __syncthreads();
+    }
     const int ngroups = T.ngroups;
+    const Fma F;
 
     for (int64_t w0 = ((int64_t)blockIdx.x * wpc + wib) * PPW; w0 < nb; w0 += (int64_t)gridDim.x * wpc * PPW) {
         const int64_t slot = w0 + sub;
         const bool valid = slot < nb;
         int32_t word = valid ? S.gst[slot] : 0x11111111;
-        const double* G = S.gram + (valid ? slot : 0) * S.gstride;
+        const double* __restrict__ G = S.gram + (valid ? slot : 0) * S.gstride;
+        int tab0 = 0;
         for (int g = 0; g < ngroups; ++g) {
             const int n = T.gn[g];
             const int nrhs = S.nrhs[g];
@@ -485,62 +506,77 @@ __global__ void __launch_bounds__(kQrWarps * 32) qr_kernel(AsmArgs a, Split S, i
             double* Z = R + n * ncol;     // solutions, n x nrhs
             const bool active = valid && group_status(word, g) == ST_OK;
             // R = [A | b...]
-            for (int e = l; e < n * ncol; e += LPP) {
-                const int i = e / ncol, j = e - i * ncol;
+            if (WS || !S.qtab) {
+                for (int e = l; e < n * n; e += LPP) {
+                    const int i = e / n, j = e - i * n;
+                    const int ui = T.gidx[g][i], uj = T.gidx[g][j];
+                    R[i * ldr + j] = active ? G[T.upair[min(ui, uj)][max(ui, uj)]] : 0.0;
+                }
+            } else {
+                const int ne = n * (n + 1) / 2;
+#pragma unroll 4
+                for (int e = l; e < ne; e += LPP) {
+                    const uint32_t t = tab[tab0 + e];
+                    const int i = (int)(t >> 8) & 255, j = (int)t & 255;
+                    const double v = active ? G[t >> 16] : 0.0;
+                    R[i * ldr + j] = v;
+                    R[j * ldr + i] = v;
+                }
+                tab0 += ne;
+            }
+            for (int e = l; e < n * nrhs; e += LPP) {
+                const int i = e / nrhs, r = e - i * nrhs;
                 double v = 0.0;
                 if (active) {
-                    if (j < n) {
-                        const int ui = T.gidx[g][i], uj = T.gidx[g][j];
-                        v = G[T.upair[min(ui, uj)][max(ui, uj)]];
-                    } else if (S.vjp) {
+                    if (S.vjp) {
                         // b~ = sum_o gbar_o b_o, then s
-                        if (j == n) {
-                            for (int r = 0; r < T.nout_rhs[g]; ++r)
-                                v += a.gbar[(int64_t)T.out_of_rhs[g][r] * a.n + b0 + slot] * T.b_out[g][r][i];
+                        if (r == 0) {
+                            for (int o = 0; o < T.nout_rhs[g]; ++o)
+                                v += a.gbar[(int64_t)T.out_of_rhs[g][o] * a.n + b0 + slot] * T.b_out[g][o][i];
                         } else {
                             v = G[S.npairs + T.gidx[g][i]];
                         }
                     } else {
-                        v = fast ? T.b_out[g][j - n][i] : T.b_term[g][j - n][i];
+                        v = fast ? T.b_out[g][r][i] : T.b_term[g][r][i];
                     }
                 }
-                R[i * ldr + j] = v;
+                R[i * ldr + n + r] = v;
             }
             for (int i = l; i < n; i += LPP) perm[i] = i;
             __syncwarp();
             bool dead = !active;
-            for (int kk = 0; kk < n; ++kk) {
-                // column norms of the trailing block, pivot = first largest
-                double best = -1.0;
-                int bidx = 0x7fffffff;
-                for (int j = kk + ((l - kk) & (LPP - 1)); j < n; j += LPP) {
-                    double sn = 0.0;
-                    for (int i = kk; i < n; ++i) sn = fma(R[i * ldr + j], R[i * ldr + j], sn);
-                    if (sn > best) {
-                        best = sn;
-                        bidx = j;
-                    }
+            // The next pivot of this lane's columns: first largest squared norm
+            // of the trailing block.  A norm is >= 0 or NaN, so the bits order
+            // the values and a NaN counts below everything (key -1).
+            long long best = -1;
+            int bidx = 0x7fffffff;
+            auto offer = [&](double sn, int j) {
+                long long key = (long long)(((unsigned long long)dhi(sn) << 32) | dlo(sn));
+                if (key > 0x7ff0000000000000ll || key < 0) key = -1;
+                if (key > best) {
+                    best = key;
+                    bidx = j;
                 }
+            };
+            for (int j = l; j < n; j += LPP) {
+                double sn = 0.0;
+                for (int i = 0; i < n; ++i) sn = fma(R[i * ldr + j], R[i * ldr + j], sn);
+                offer(sn, j);
+            }
+            for (int kk = 0; kk < n; ++kk) {
 #pragma unroll
                 for (int o = LPP / 2; o > 0; o >>= 1) {
-                    double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                    int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
+                    const long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+                    const int oi = __shfl_xor_sync(0xffffffffu, bidx, o);
                     if (ob > best || (ob == best && oi < bidx)) {
                         best = ob;
                         bidx = oi;
                     }
                 }
                 const int piv = (bidx == 0x7fffffff) ? kk : bidx;
-                // sigma = the pivot column's norm (NaN when all norms were NaN)
-                double sigma;
-                if (bidx == 0x7fffffff) {
-                    double sn = 0.0;
-                    for (int i = kk; i < n; ++i) sn = fma(R[i * ldr + kk], R[i * ldr + kk], sn);
-                    sigma = sn;
-                } else {
-                    sigma = best;
-                }
-                dead |= !(sigma > 0.0);
+                // sigma: the pivot column's squared norm (NaN when all were)
+                const double sigma = __hiloint2double((int)(best >> 32), (int)best);
+                dead |= best <= 0;
                 if (piv != kk) {
                     for (int i = l; i < n; i += LPP) {
                         const double t0 = R[i * ldr + kk];
@@ -556,28 +592,89 @@ __global__ void __launch_bounds__(kQrWarps * 32) qr_kernel(AsmArgs a, Split S, i
                 __syncwarp();
                 const double alpha = R[kk * ldr + kk];
                 const double nr = sqrt(sigma);
-                const double beta = (alpha >= 0.0) ? -nr : nr;
-                const double den = alpha - beta;
-                const double tau = (beta - alpha) / beta;
+                const double beta = (!(dhi(alpha) >> 31) || is_zero(alpha)) ? -nr : nr;  // alpha >= 0
+                const double den = F.add(alpha, -beta);
+                // 1 / den on even lanes beside 1 / beta on odd ones
+                double rden, rbeta;
+                if constexpr (LPP == 1) {
+                    rden = __drcp_rn(den);
+                    rbeta = __drcp_rn(beta);
+                } else {
+                    const double rc = __drcp_rn((l & 1) ? beta : den);
+                    rden = __shfl_sync(0xffffffffu, rc, lane & ~1);
+                    rbeta = __shfl_sync(0xffffffffu, rc, lane | 1);
+                }
+                const double tau = F.quot(-den, beta, rbeta);  // (beta - alpha) / beta
                 __syncwarp();
-                for (int i = kk + 1 + l; i < n; i += LPP) R[i * ldr + kk] = R[i * ldr + kk] / den;
+                for (int i = kk + 1 + l; i < n; i += LPP) R[i * ldr + kk] = F.quot(R[i * ldr + kk], den, rden);
                 __syncwarp();
                 if (l == 0) R[kk * ldr + kk] = beta;
-                for (int j = kk + 1 + l; j < ncol; j += LPP) {
-                    double sv = R[kk * ldr + j];
-                    for (int i = kk + 1; i < n; ++i) sv = fma(R[i * ldr + kk], R[i * ldr + j], sv);
-                    sv = sv * tau;
-                    R[kk * ldr + j] = R[kk * ldr + j] - sv;
-                    for (int i = kk + 1; i < n; ++i) R[i * ldr + j] = fma(-sv, R[i * ldr + kk], R[i * ldr + j]);
+                best = -1;
+                bidx = 0x7fffffff;
+                const double* v = R + (kk + 1) * ldr + kk;
+                const int m = n - kk - 1;
+                // the reflection of columns kk + 1 .., two of this lane's at a
+                // time, and the squared norms the next pivot is chosen by
+                int j = kk + 1 + l;
+                for (; j + LPP < ncol; j += 2 * LPP) {
+                    double* c0 = R + kk * ldr + j;
+                    double* c1 = c0 + LPP;
+                    double s0 = c0[0], s1 = c1[0];
+                    c0 += ldr;
+                    c1 += ldr;
+#pragma unroll 4
+                    for (int i = 0; i < m; ++i) {
+                        const double vi = v[i * ldr];
+                        s0 = fma(vi, c0[i * ldr], s0);
+                        s1 = fma(vi, c1[i * ldr], s1);
+                    }
+                    s0 = F.mul(s0, tau);
+                    s1 = F.mul(s1, tau);
+                    c0[-ldr] = F.add(c0[-ldr], -s0);
+                    c1[-ldr] = F.add(c1[-ldr], -s1);
+                    double n0 = 0.0, n1 = 0.0;
+#pragma unroll 4
+                    for (int i = 0; i < m; ++i) {
+                        const double vi = v[i * ldr];
+                        const double x0 = fma(-s0, vi, c0[i * ldr]), x1 = fma(-s1, vi, c1[i * ldr]);
+                        c0[i * ldr] = x0;
+                        c1[i * ldr] = x1;
+                        n0 = fma(x0, x0, n0);
+                        n1 = fma(x1, x1, n1);
+                    }
+                    if (j < n) offer(n0, j);
+                    if (j + LPP < n) offer(n1, j + LPP);
+                }
+                if (j < ncol) {
+                    double* c0 = R + kk * ldr + j;
+                    double s0 = c0[0];
+                    c0 += ldr;
+#pragma unroll 4
+                    for (int i = 0; i < m; ++i) s0 = fma(v[i * ldr], c0[i * ldr], s0);
+                    s0 = F.mul(s0, tau);
+                    c0[-ldr] = F.add(c0[-ldr], -s0);
+                    double n0 = 0.0;
+#pragma unroll 4
+                    for (int i = 0; i < m; ++i) {
+                        const double x0 = fma(-s0, v[i * ldr], c0[i * ldr]);
+                        c0[i * ldr] = x0;
+                        n0 = fma(x0, x0, n0);
+                    }
+                    if (j < n) offer(n0, j);
                 }
                 __syncwarp();
             }
-            // back substitution, right-hand sides split over the lanes
+            // back substitution, right-hand sides split over the lanes; the
+            // diagonal's reciprocals, a lane each, over row n - 1 of the
+            // reflections (not needed any more)
+            for (int i = l; i < n - 1; i += LPP) R[(n - 1) * ldr + i] = __drcp_rn(R[i * ldr + i]);
+            const double rlast = __drcp_rn(R[(n - 1) * ldr + n - 1]);
+            __syncwarp();
             for (int r = l; r < nrhs; r += LPP) {
                 for (int i = n - 1; i >= 0; --i) {
                     double sv = R[i * ldr + n + r];
                     for (int j = i + 1; j < n; ++j) sv = fma(-R[i * ldr + j], Z[j * nrhs + r], sv);
-                    Z[i * nrhs + r] = sv / R[i * ldr + i];
+                    Z[i * nrhs + r] = F.quot(sv, R[i * ldr + i], i == n - 1 ? rlast : R[(n - 1) * ldr + i]);
                 }
             }
             __syncwarp();
@@ -907,8 +1004,9 @@ cudaError_t launch_gram(const AsmArgs& a, const Split& S, int64_t b0, int64_t b1
 // lanes, 64-bit accesses) fall on distinct shared-memory banks.
 int qr_pstride(const Split& S, int lpp) { return S.qwords + ((lpp - S.qwords) & 15); }
 
-size_t qr_bytes(const Split& S, int lpp) {
-    return (size_t)kQrWarps * (32 / lpp) * (qr_pstride(S, lpp) * sizeof(double) + S.nmax * sizeof(int));
+size_t qr_bytes(const Split& S, int lpp, bool table = true) {
+    return (size_t)kQrWarps * (32 / lpp) * (qr_pstride(S, lpp) * sizeof(double) + S.nmax * sizeof(int)) +
+           (table ? (size_t)S.qtab * sizeof(uint32_t) : 0);
 }
 
 // CTAs per SM of the QR with its work space in global memory (one warp and
@@ -919,13 +1017,15 @@ template <int LPP>
 cudaError_t launch_qr(const AsmArgs& a, Split S, int64_t b0, int64_t nb, cudaStream_t s) {
     constexpr int PPW = 32 / LPP;
     S.pstride = qr_pstride(S, LPP);
+    // without the table of Gram entries where it is what does not fit
+    if (qr_bytes(S, LPP) > (size_t)smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024)) S.qtab = 0;
     if (S.qws) {
         const int64_t grid = std::min<int64_t>((int64_t)num_sms() * kQrGlobalPerSm, nb);
-        qr_kernel<LPP><<<(unsigned)std::max<int64_t>(grid, 1), 32, 0, s>>>(a, S, b0, nb);
+        qr_kernel<LPP, true><<<(unsigned)std::max<int64_t>(grid, 1), 32, 0, s>>>(a, S, b0, nb);
         return cudaGetLastError();
     }
     const size_t bytes = qr_bytes(S, LPP);
-    auto kern = qr_kernel<LPP>;
+    auto kern = qr_kernel<LPP, false>;
     int grid = 0;
     cudaError_t e = persistent(kern, kQrWarps * 32, bytes, (int64_t)kQrWarps * PPW, nb, grid);
     if (e != cudaSuccess) return e;
@@ -953,17 +1053,23 @@ cudaError_t launch_weights(const AsmArgs& a, const Split& S, int64_t b0, int64_t
     return cudaGetLastError();
 }
 
-// lanes per particle of the QR: the fewest that still leave >= 6 warps per SM
-// resident within the shared-memory budget (on the 128^3 gradient+Laplacian
-// cloud 4 lanes / 6 warps beat 8 lanes / 12 warps and 2 lanes / 2 warps)
-int qr_lanes_auto(const Split& S) {
+// Lanes per particle of the QR: the fewest from two on that still leave >= 6
+// warps per SM resident within the shared-memory budget, then up to eight while
+// the particles give the GPU less than a warp per scheduler.  Measured (whole
+// fast assembly, ms, for 1 / 2 / 4 / 8 / 16 lanes): 60^3 Gradient + Laplacian 25.5
+// / 19.9 / 17.4 / 18.9 / 22.7; 2D Laplacian, 65,536 particles 1.01 / 0.95 / 1.04 /
+// 1.14 / 1.39, 4,096 particles 0.274 / 0.249 / 0.237 / 0.232 / 0.243; uneven 2D
+// cloud, 2e5 particles, five operators 4.07 / 3.58 / 3.78 / 4.43 / 5.57.
+int qr_lanes_auto(const Split& S, int64_t nb) {
     const int per_sm = smem_attr(cudaDevAttrMaxSharedMemoryPerMultiprocessor, 228 * 1024);
     const int per_block = smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024);
-    for (int lpp : {1, 2, 4, 8, 16}) {
+    for (int lpp : {2, 4, 8, 16}) {
         const size_t b = qr_bytes(S, lpp);
         if (b > (size_t)per_block) continue;
         const int blocks = (int)(per_sm / (b + 1024));
-        if (blocks * kQrWarps >= 6) return lpp;
+        if (blocks * kQrWarps < 6) continue;
+        while (lpp < 8 && nb * lpp / 32 < (int64_t)num_sms() * 4) lpp *= 2;
+        return lpp;
     }
     return 32;
 }
@@ -1074,6 +1180,7 @@ Split make_split(const AsmTables& h, int flags, bool vjp = false) {
         S.c_off[g] = off;
         off += n * S.nrhs[g];
         S.nmax = std::max(S.nmax, n);
+        S.qtab += n * (n + 1) / 2;
         S.nrmax = std::max(S.nrmax, S.nrhs[g]);
         S.qwords = std::max(S.qwords, n * (n + S.nrhs[g]) + n * S.nrhs[g]);
     }
@@ -1114,7 +1221,7 @@ int64_t vjp_scratch_bytes(const AsmTables& h, int maxk) {
 
 int64_t assembly_qr_ws_bytes(const AsmTables& h, int flags) {
     Split S = make_split(h, flags);
-    if (qr_bytes(S, 32) <= (size_t)smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024)) return 0;
+    if (qr_bytes(S, 32, false) <= (size_t)smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024)) return 0;
     const int64_t slots = (int64_t)num_sms() * kQrGlobalPerSm;
     return slots * ((int64_t)qr_pstride(S, 32) * (int64_t)sizeof(double) + (int64_t)S.nmax * (int64_t)sizeof(int));
 }
@@ -1177,13 +1284,13 @@ cudaError_t assemble(const AsmArgs& a, const AsmTables& h, cudaStream_t s) {
         S.gst = reinterpret_cast<int32_t*>(S.usc + nb * S.ustride);
     }
     int lpp = a.qr_lanes;
-    if (lpp != 1 && lpp != 2 && lpp != 4 && lpp != 8 && lpp != 16 && lpp != 32) lpp = qr_lanes_auto(S);
+    if (lpp != 1 && lpp != 2 && lpp != 4 && lpp != 8 && lpp != 16 && lpp != 32) lpp = qr_lanes_auto(S, std::min(a.n, nb));
     if (a.qws) {
         // large bases: one warp per particle, the work space in global memory
         lpp = 32;
         S.qws = a.qws;
         S.qperm = reinterpret_cast<int*>(a.qws + (int64_t)num_sms() * kQrGlobalPerSm * qr_pstride(S, 32));
-    } else if (qr_bytes(S, lpp) > (size_t)smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024)) {
+    } else if (qr_bytes(S, lpp, false) > (size_t)smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024)) {
         // a lane grouping whose work space does not fit is refused before any launch
         return cudaErrorInvalidConfiguration;
     }
@@ -1205,8 +1312,8 @@ cudaError_t vjp_entries(const AsmArgs& a, const AsmTables& h, cudaStream_t s) {
     S.usc = S.scale + nb * 4;
     S.gst = reinterpret_cast<int32_t*>(S.usc + nb * S.ustride);
     int lpp = a.qr_lanes;
-    if (lpp != 1 && lpp != 2 && lpp != 4 && lpp != 8 && lpp != 16 && lpp != 32) lpp = qr_lanes_auto(S);
-    if (qr_bytes(S, lpp) > (size_t)smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024))
+    if (lpp != 1 && lpp != 2 && lpp != 4 && lpp != 8 && lpp != 16 && lpp != 32) lpp = qr_lanes_auto(S, std::min(a.n, nb));
+    if (qr_bytes(S, lpp, false) > (size_t)smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024))
         lpp = 32;  // a lane grouping chosen for the assembly's right-hand sides
     if (h.dim == 3) return vjp_run<3>(a, h, S, lpp, s);
     if (h.dim == 2) return vjp_run<2>(a, h, S, lpp, s);
