@@ -162,34 +162,36 @@ __global__ void transpose_outputs_kernel(const int64_t* __restrict__ tidx, int64
     }
 }
 
-// grad x_i -= sum over the entries pointing at i of their gradients: a warp
-// per transposed row, the row's own sums are in grad already (vjp_entries)
+// grad x_i -= sum over the entries pointing at i of their gradients: eight lanes
+// per transposed row (the row's own sums are in grad already, vjp_entries)
 template <int DIM>
 __global__ void __launch_bounds__(256) vjp_gather_kernel(const int64_t* __restrict__ trow,
                                                          const int64_t* __restrict__ tidx, int64_t n,
                                                          const double* __restrict__ G, double* __restrict__ grad) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += nw) {
+    const int sub = threadIdx.x & 7;
+    const int64_t nr = ((int64_t)gridDim.x * blockDim.x) >> 3;
+    const int64_t i0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
+    for (int64_t w = i0 - ((threadIdx.x >> 3) & 3); w < n; w += nr) {  // (warp-uniform)
+        const int64_t i = w + ((threadIdx.x >> 3) & 3);
         double s[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) s[d] = 0.0;
-        const int64_t e = trow[i + 1];
-        for (int64_t t = trow[i] + lane; t < e; t += 32) {
+        const int64_t e = i < n ? trow[i + 1] : 0;
+        for (int64_t t = (i < n ? trow[i] : 0) + sub; t < e; t += 8) {
             const int64_t j = tidx[t];
 #pragma unroll
             for (int d = 0; d < DIM; ++d) s[d] += G[j * DIM + d];
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
             for (int d = 0; d < DIM; ++d) s[d] += __shfl_xor_sync(0xffffffffu, s[d], o);
-        if (lane < DIM) {
+        if (i < n && sub < DIM) {
             double v = s[0];
 #pragma unroll
             for (int d = 1; d < DIM; ++d)
-                if (lane == d) v = s[d];
-            grad[i * DIM + lane] -= v;
+                if (sub == d) v = s[d];
+            grad[i * DIM + sub] -= v;
         }
     }
 }
@@ -268,7 +270,7 @@ cudaError_t transpose_outputs(const int64_t* tidx, int64_t nnz, int nout, const 
 cudaError_t vjp_gather(const int64_t* trow, const int64_t* tidx, int64_t n, int dim, const double* gentry,
                        double* grad, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    const int grid = grid_for(n * 32);
+    const int grid = grid_for(n * 8);
     if (dim == 3)
         vjp_gather_kernel<3><<<grid, 256, 0, s>>>(trow, tidx, n, gentry, grad);
     else if (dim == 2)

@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(256) apply_terms_f64_kernel(TermsArgs a) {
 // lines a load), so the products stay on the pipe, as dfmas: 64^3 periodic 128
 // us with dmul and dadd, 121 us; on the integer pipes they cost the occupancy
 // that hides the loads (146 us).
-__global__ void __launch_bounds__(256, 6) p2p_f64_kernel(int64_t n, const int64_t* __restrict__ rowptr,
+__global__ void __launch_bounds__(256) p2p_f64_kernel(int64_t n, const int64_t* __restrict__ rowptr,
                                                       const int32_t* __restrict__ cols, const double* __restrict__ K,
                                                       const double* __restrict__ eip, int ncomp,
                                                       const double* __restrict__ f, double* __restrict__ out) {
@@ -174,28 +174,25 @@ __global__ void __launch_bounds__(256, 6) p2p_f64_kernel(int64_t n, const int64_
     for (int64_t base = (int64_t)blockIdx.x * 256; base < n; base += (int64_t)gridDim.x * 256) {
         const int64_t p = row_by_length(base, n, rowptr, s_len, s_row);
         if (p >= n) continue;
-        const int64_t b = rowptr[p];
-        const int len = (int)(rowptr[p + 1] - b);
-        const int32_t* __restrict__ cr = cols + b;
-        const double* __restrict__ Kr = K + b;
+        const int64_t b = rowptr[p], e = rowptr[p + 1];
         for (int c = 0; c < ncomp; ++c) {
             double D = 0.0;
-            int j = 0;
+            int64_t j = b;
             // 4 entries in flight, summed in row order
-            for (; j + 4 <= len; j += 4) {
+            for (; j + 4 <= e; j += 4) {
                 int32_t q[4];
                 double k[4], fq[4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-                    q[u] = cr[j + u];
-                    k[u] = Kr[j + u];
+                    q[u] = cols[j + u];
+                    k[u] = K[j + u];
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) fq[u] = f[(int64_t)q[u] * ncomp + c];
 #pragma unroll
                 for (int u = 0; u < 4; ++u) D = F.add(F.mul(fq[u], k[u]), D);
             }
-            for (; j < len; ++j) D = F.add(F.mul(f[(int64_t)cr[j] * ncomp + c], Kr[j]), D);
+            for (; j < e; ++j) D = F.add(F.mul(f[(int64_t)cols[j] * ncomp + c], K[j]), D);
             out[p * ncomp + c] = eip[p] * D;
         }
     }

@@ -13,9 +13,9 @@
 // the chain rule formed every derivative monomial from powers, per basis
 // function and group (3D Gradient + Laplacian: about 580 FP64 instructions per
 // 32 entries).  Here the monomials come from the monomial program (16
-// products), the coefficient of each union monomial is summed over the groups
-// first and meets its derivatives, which are other slots of the same program,
-// once: about 200 per 32 entries.
+// products, on the integer pipes), the coefficient of each union monomial is
+// summed over the groups first and meets its derivatives, which are other slots
+// of the same program, once: about 165 per 32 entries.
 
 struct ChainShared {
     ProgShared P;
@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(256) vjp_chain_kernel(AsmArgs a, Split S, int6
             X.guse[T.gidx[g][i]][g] = (unsigned char)(i + 1);
         }
     __syncthreads();
+    const Fma F;
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     double* Cs = smem + (size_t)wib * (S.cstride + (S.nslots + 2 * ngroups) * 32);
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(256) vjp_chain_kernel(AsmArgs a, Split S, int6
         }
         for (int e = lane; e < S.cstride; e += 32) Cs[e] = S.coef[slot * S.cstride + e];
         __syncwarp();
-        const double ieps = 1.0 / a.eps[p];
+        const double ieps = S.scale[slot * 4 + 1];
         // d Phi / d eps from e = eps^-|alpha|: -|alpha| e s^T a~ / eps
         double Dsc = 0.0;
         const double* sv = S.gram + slot * S.gstride + S.npairs;
@@ -100,9 +101,15 @@ __global__ void __launch_bounds__(256) vjp_chain_kernel(AsmArgs a, Split S, int6
                 gu[d] = 0.0;
             }
             const double E = Ur[DIM * S.maxk + q];
-            const double om = E * E;
-            const double cq = a.f[a.cols[beg + q]] - fp;
-            monomials<DIM>(u, V, X.P, nprog, lane);
+            const double om = F.prod(E, E);
+            const double cq = F.add(a.f[a.cols[beg + q]], -fp);
+            bool unit = true;
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) unit = unit && unit_range_or_zero(u[d]);
+            if (unit)
+                monomials_int<DIM>(u, V, X.P, nprog, lane);
+            else
+                monomials<DIM>(u, V, X.P, nprog, lane);
             double ga = 0.0;
             for (int g = 0; g < ngroups; ++g) {
                 const double* C = Cs + S.c_off[g];
@@ -113,11 +120,11 @@ __global__ void __launch_bounds__(256) vjp_chain_kernel(AsmArgs a, Split S, int6
                     va = fma(v, C[2 * i], va);
                     vl = fma(v, C[2 * i + 1], vl);
                 }
-                const double eo = a.eip_group[(int64_t)g * a.n + p] * om;
-                const double c1 = eo * (cq - vl);
+                const double eo = F.prod(a.eip_group[(int64_t)g * a.n + p], om);
+                const double c1 = F.prod(eo, F.add(cq, -vl));
                 ga = fma(va, c1, ga);
                 CC[(2 * g) * 32 + lane] = c1;
-                CC[(2 * g + 1) * 32 + lane] = -(eo * va);
+                CC[(2 * g + 1) * 32 + lane] = -F.prod(eo, va);
             }
             for (int j = 0; j < nu; ++j) {
                 double beta = 0.0;
@@ -132,21 +139,22 @@ __global__ void __launch_bounds__(256) vjp_chain_kernel(AsmArgs a, Split S, int6
                 for (int d = 0; d < DIM; ++d) {
                     const int e = X.uexp[j][d];
                     if (e == 0) continue;
-                    const double b = e == 1 ? beta : beta * kSmallInt[e];
+                    const double b = e == 1 ? beta : F.prod(beta, kSmallInt[e]);
                     gu[d] = fma(b, V[X.dslot[j][d] * 32 + lane], gu[d]);
                 }
             }
-            ga = -2.0 * ga;
+            ga = F.add(-ga, -ga);
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {
                 gu[d] = fma(ga, u[d], gu[d]);
                 gsum = fma(gu[d], u[d], gsum);
-                Gp[q * DIM + d] = gu[d] * ieps;
+                Gp[q * DIM + d] = F.prod(gu[d], ieps);
             }
         }
         // the eps terms, along sign(x_pq) (u has x_pq's sign); without them
         // for a fixed eps
         const double dd = a.eps_fixed ? 0.0 : warp_sum(Dsc - gsum) * ieps / ((double)k * a.h_over_eps);
+        const double dz = 0.0 * dd;  // (NaN where dd is not finite)
         double own[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; ++d) own[d] = 0.0;
@@ -154,10 +162,10 @@ __global__ void __launch_bounds__(256) vjp_chain_kernel(AsmArgs a, Split S, int6
 #pragma unroll
             for (int d = 0; d < DIM; ++d) {
                 const double o = Ur[d * S.maxk + q];
-                const double sg = (o > 0.0) ? dd : ((o < 0.0) ? -dd : 0.0 * dd);
-                const double v = Gp[q * DIM + d] + sg;
+                const double sg = is_zero(o) ? dz : ((dhi(o) >> 31) ? -dd : dd);
+                const double v = F.add(Gp[q * DIM + d], sg);
                 Gp[q * DIM + d] = v;
-                own[d] += v;
+                own[d] = F.add(v, own[d]);
             }
         }
 #pragma unroll
