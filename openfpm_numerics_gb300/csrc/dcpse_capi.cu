@@ -229,6 +229,7 @@ struct dcpse_plan_s {
     AsmTables* htab = nullptr;  // host copy
     AsmTables* dtab = nullptr;  // device copy
     cudaStream_t stream = nullptr;
+    bool stream_changed = false;  // since the last assembly: earlier work may run on another stream
     bool has_box = false;
     double lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};
     int per[3] = {0, 0, 0};
@@ -388,7 +389,33 @@ struct dcpse_plan_s {
     double* sell_w64 = nullptr;  // FP64 summed weights on the same layout (with w64)
     int64_t sell_total = 0;
     bool sell_no_room = false;  // the copy did not fit in device memory: CSR kernels only
+    // The layout (rows, slices, columns) belongs to the list, the weights on it
+    // to an assembly: a re-assembly keeps the layout and, as spares, the
+    // buffers its weights go into again (80^3: rebuilding it took 0.6 ms and
+    // four host synchronisations per assembly).
+    float *spare_w = nullptr, *spare_r32 = nullptr;
+    double* spare_w64 = nullptr;
+    void* spare_r = nullptr;
+    void drop_sell_weights(bool f32, bool f64) {
+        auto keep = [](auto& live, auto& spare, bool wanted) {
+            if (live && wanted && !spare)
+                spare = live;
+            else if (live)
+                cudaFree((void*)live);
+            live = nullptr;
+            if (!wanted && spare) {
+                cudaFree((void*)spare);
+                spare = nullptr;
+            }
+        };
+        keep(sell_w, spare_w, f32);
+        keep(sell_r32, spare_r32, f32);
+        keep(sell_r, spare_r, f32);
+        keep(sell_w64, spare_w64, f64);
+        sell_no_room = false;
+    }
     void free_sell() {
+        drop_sell_weights(false, false);
         sell_perm = nullptr;
         dfree(sell_inv);
         dfree(fperm);
@@ -396,13 +423,7 @@ struct dcpse_plan_s {
         dfree(sell_row);
         dfree(sell_off);
         dfree(sell_cols);
-        dfree(sell_w);
-        dfree(sell_w64);
-        if (sell_r) cudaFree(sell_r);
-        sell_r = nullptr;
-        dfree(sell_r32);
         sell_total = 0;
-        sell_no_room = false;
     }
     void free_assembly() {
         free_sell();
@@ -887,6 +908,7 @@ int dcpse_plan_destroy(dcpse_plan_t* P) {
 
 int dcpse_plan_set_stream(dcpse_plan_t* P, void* stream) {
     if (int rc = check_plan(P)) return rc;
+    if (P->stream != (cudaStream_t)stream) P->stream_changed = true;
     P->stream = (cudaStream_t)stream;
     return DCPSE_OK;
 }
@@ -1292,7 +1314,14 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
     if (!(flags & DCPSE_STORE_TERMS_F64)) dfree(P->k_term);
     if ((flags & DCPSE_STORE_OUT_F64) && !P->w64) DCPSE_CK(dalloc(&P->w64, (size_t)P->nout * nnz));
     if (!(flags & DCPSE_STORE_OUT_F64)) dfree(P->w64);
-    P->free_sell();  // the FP32 weights are rewritten
+    // the weights are rewritten (a surface operator's list, too): not while
+    // an apply on the plan's previous stream still reads them
+    if (P->stream_changed) DCPSE_CK(cudaDeviceSynchronize());
+    P->stream_changed = false;
+    if (P->surface())
+        P->free_sell();
+    else
+        P->drop_sell_weights((flags & DCPSE_STORE_OUT_F32) != 0, (flags & DCPSE_STORE_OUT_F64) != 0);
     // so are the field VJP's row sums and transposed weights
     dfree(P->rowsum);
     P->rowsum_prec = -1;
@@ -2059,6 +2088,14 @@ int ensure_sell_layout(dcpse_plan_t* P) {
     return DCPSE_OK;
 }
 
+// the spare buffer of an earlier assembly on the same layout, or a new one
+extern "C++" template <typename T>
+cudaError_t spare_or(T*& live, T*& spare, size_t count) {
+    if (!spare) return dalloc(&live, count);
+    std::swap(live, spare);
+    return cudaSuccess;
+}
+
 // One set of weights on the sliced layout: a failed allocation leaves it
 // absent (the CSR kernels serve), other errors fail.
 extern "C++" template <typename Alloc, typename Fill, typename Release>
@@ -2081,7 +2118,8 @@ int ensure_sell(dcpse_plan_t* P) {
     if (int rc = ensure_sell_layout(P)) return rc;
     if (!P->sell_cols) return DCPSE_OK;
     return sell_stream(
-        P, "sliced ELL weights: ", [&] { return dalloc(&P->sell_w, (size_t)P->nout * P->sell_total + kPad); },
+        P, "sliced ELL weights: ",
+        [&] { return spare_or(P->sell_w, P->spare_w, (size_t)P->nout * P->sell_total + kPad); },
         [&] {
             return sell_fill(P->rowptr, P->cols, P->w32, nullptr, P->nnz, P->nout, P->n, P->two_set() ? 0 : 1,
                              P->sell_row, P->sell_off, P->sell_total, nullptr, P->sell_w, nullptr, P->stream,
@@ -2098,7 +2136,7 @@ int ensure_sell64(dcpse_plan_t* P) {
     if (!P->sell_cols) return DCPSE_OK;
     return sell_stream(
         P, "sliced ELL FP64 weights: ",
-        [&] { return dalloc(&P->sell_w64, (size_t)P->nout * P->sell_total + kPad); },
+        [&] { return spare_or(P->sell_w64, P->spare_w64, (size_t)P->nout * P->sell_total + kPad); },
         [&] {
             return sell_fill64(P->rowptr, P->w64, P->nnz, P->nout, P->n, P->sell_row, P->sell_off, P->sell_total,
                                P->sell_w64, P->stream, P->sell_perm);
@@ -2112,7 +2150,13 @@ int ensure_sell_resid(dcpse_plan_t* P) {
     if (P->sell_r || !P->sell_w || !P->r16) return DCPSE_OK;
     return sell_stream(
         P, "sliced ELL residuals: ",
-        [&] { return cudaMalloc(&P->sell_r, ((size_t)P->nout * P->sell_total + kPad) * 2); },
+        [&] {
+            if (P->spare_r) {
+                std::swap(P->sell_r, P->spare_r);
+                return cudaSuccess;
+            }
+            return cudaMalloc(&P->sell_r, ((size_t)P->nout * P->sell_total + kPad) * 2);
+        },
         [&] {
             return sell_fill(P->rowptr, P->cols, nullptr, P->r16, P->nnz, P->nout, P->n, P->two_set() ? 0 : 1,
                              P->sell_row, P->sell_off, P->sell_total, nullptr, nullptr, P->sell_r, P->stream,
@@ -2130,7 +2174,7 @@ int ensure_sell_pair(dcpse_plan_t* P) {
     if (P->sell_r32 || !P->sell_w || !P->r32) return DCPSE_OK;
     return sell_stream(
         P, "sliced ELL weight pairs: ",
-        [&] { return dalloc(&P->sell_r32, (size_t)P->nout * P->sell_total + kPad); },
+        [&] { return spare_or(P->sell_r32, P->spare_r32, (size_t)P->nout * P->sell_total + kPad); },
         [&] {
             // the residuals take the weight streams' path of the fill
             return sell_fill(P->rowptr, P->cols, P->r32, nullptr, P->nnz, P->nout, P->n, P->two_set() ? 0 : 1,
