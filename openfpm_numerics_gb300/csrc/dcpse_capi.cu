@@ -12,7 +12,10 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
+#include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "dcpse_internal.h"
@@ -165,16 +168,158 @@ constexpr int64_t kPad = 8;
 // batches of particles (the result does not depend on the batch size).
 constexpr int64_t kAsmScratchBytes = int64_t(512) << 20;
 
-template <typename T>
-cudaError_t dalloc(T** p, size_t count) {
-    *p = nullptr;
-    if (count == 0) count = 1;
-    return cudaMalloc((void**)p, count * sizeof(T));
+// Device memory of the plans.  A freed block is kept for the next request of
+// about its size instead of going back to the driver, whose cudaMalloc and
+// cudaFree cost 10 us to 1 ms each (a neighbour build makes 14 of each, an
+// operator update of 4,096 particles spent 0.6 of its 1.0 ms there).  Shared by
+// all plans and threads of the process, since an operator update builds its list
+// on a plan of its own.  Bounded: at most kPoolBytes of free blocks per process,
+// given back when a request cannot be met and when the last plan is destroyed.
+// cudaFree waits for the device; here a block is handed out again only after a
+// device synchronisation later than its release, so whatever stream or thread
+// still used it when it was freed has finished.
+thread_local cudaStream_t t_plan_stream = nullptr;  // stream of the plan this thread works on (check_plan)
+
+class DevicePool {
+public:
+    cudaError_t alloc(void** p, size_t want) {
+        *p = nullptr;
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        size_t bytes = rounded(want);
+        unsigned long long wait = 0;
+        {
+            std::lock_guard<std::mutex> lock(m_);
+            if (take(p, dev, bytes, synced_[dev])) return cudaSuccess;
+            if (find(dev, bytes, ~0ull) != free_.end()) wait = stamp_;
+        }
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (wait && (cudaStreamIsCapturing(t_plan_stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) {
+            cudaGetLastError();
+            wait = 0;  // inside a stream capture: as without a pool
+        }
+        if (wait) {
+            // released, but perhaps still in use: after a synchronisation not
+            if (cudaDeviceSynchronize() == cudaSuccess) {
+                std::lock_guard<std::mutex> lock(m_);
+                synced_[dev] = std::max(synced_[dev], wait);
+                if (take(p, dev, bytes, synced_[dev])) return cudaSuccess;
+            }
+        }
+        e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            release();
+            bytes = want;
+            e = cudaMalloc(p, bytes);
+        }
+        if (e == cudaSuccess) {
+            std::lock_guard<std::mutex> lock(m_);
+            live_[*p] = Block{bytes, dev, 0};
+        } else {
+            *p = nullptr;
+        }
+        return e;
+    }
+    void free(void* p) {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lock(m_);
+            auto it = live_.find(p);
+            if (it != live_.end()) {
+                Block b = it->second;
+                live_.erase(it);
+                if (cached_ + b.bytes <= kPoolBytes) {
+                    b.stamp = ++stamp_;
+                    cached_ += b.bytes;
+                    free_.emplace(b.bytes, std::make_pair(p, b));
+                    return;
+                }
+            }
+        }
+        cudaFree(p);
+    }
+    void plan_created() {
+        std::lock_guard<std::mutex> lock(m_);
+        ++plans_;
+    }
+    void plan_destroyed() {
+        bool last;
+        {
+            std::lock_guard<std::mutex> lock(m_);
+            last = --plans_ == 0;
+        }
+        if (last) release();
+    }
+    // every free block back to the driver
+    void release() {
+        std::vector<std::pair<void*, int>> blocks;
+        {
+            std::lock_guard<std::mutex> lock(m_);
+            for (auto& f : free_) blocks.emplace_back(f.second.first, f.second.second.dev);
+            free_.clear();
+            cached_ = 0;
+        }
+        for (auto& b : blocks) cudaFree(b.first);  // (any device's: pointers are unified)
+    }
+
+private:
+    static constexpr size_t kPoolBytes = size_t(4) << 30;
+    struct Block {
+        size_t bytes;
+        int dev;
+        unsigned long long stamp;  // order of the releases
+    };
+    // sixteenths of a power of two, at least 512 bytes: lists and weights of
+    // moving particles change a little in size from step to step
+    static size_t rounded(size_t want) {
+        size_t unit = 512;
+        while (unit * 32 <= want) unit *= 2;
+        return (want + unit - 1) / unit * unit;
+    }
+    using FreeMap = std::multimap<size_t, std::pair<void*, Block>>;
+    // a free block of this device of `bytes` or up to an eighth more, released
+    // before the device's last known synchronisation
+    FreeMap::iterator find(int dev, size_t bytes, unsigned long long synced) {
+        for (auto it = free_.lower_bound(bytes); it != free_.end() && it->first <= bytes + bytes / 8; ++it)
+            if (it->second.second.dev == dev && it->second.second.stamp <= synced) return it;
+        return free_.end();
+    }
+    bool take(void** p, int dev, size_t bytes, unsigned long long synced) {
+        auto it = find(dev, bytes, synced);
+        if (it == free_.end()) return false;
+        *p = it->second.first;
+        live_[*p] = it->second.second;
+        cached_ -= it->first;
+        free_.erase(it);
+        return true;
+    }
+    std::mutex m_;
+    std::unordered_map<void*, Block> live_;
+    FreeMap free_;
+    std::unordered_map<int, unsigned long long> synced_;
+    unsigned long long stamp_ = 0;
+    size_t cached_ = 0;
+    int plans_ = 0;
+};
+
+// (never destroyed: plans may outlive static destructors)
+DevicePool& pool() {
+    static DevicePool* p = new DevicePool;
+    return *p;
 }
 
 template <typename T>
+cudaError_t dalloc(T** p, size_t count) {
+    if (count == 0) count = 1;
+    return pool().alloc((void**)p, count * sizeof(T));
+}
+cudaError_t dalloc_bytes(void** p, size_t bytes) { return pool().alloc(p, bytes ? bytes : 1); }
+
+template <typename T>
 void dfree(T*& p) {
-    if (p) cudaFree((void*)p);
+    if (p) pool().free((void*)p);
     p = nullptr;
 }
 
@@ -188,6 +333,10 @@ struct KernelTimer {
 };
 
 struct dcpse_plan_s {
+    dcpse_plan_s() { pool().plan_created(); }
+    ~dcpse_plan_s() { pool().plan_destroyed(); }
+    dcpse_plan_s(const dcpse_plan_s&) = delete;
+    dcpse_plan_s& operator=(const dcpse_plan_s&) = delete;
     // optional event timing per kernel id
     bool timing = false;
     KernelTimer timers[DCPSE_K_COUNT];
@@ -401,12 +550,9 @@ struct dcpse_plan_s {
             if (live && wanted && !spare)
                 spare = live;
             else if (live)
-                cudaFree((void*)live);
+                dfree(live);
             live = nullptr;
-            if (!wanted && spare) {
-                cudaFree((void*)spare);
-                spare = nullptr;
-            }
+            if (!wanted) dfree(spare);
         };
         keep(sell_w, spare_w, f32);
         keep(sell_r32, spare_r32, f32);
@@ -433,8 +579,7 @@ struct dcpse_plan_s {
         dfree(k_term);
         dfree(w64);
         dfree(w32);
-        if (r16) cudaFree(r16);
-        r16 = nullptr;
+        dfree(r16);
         dfree(r32);
         dfree(bnd);
         dfree(blist);
@@ -687,6 +832,7 @@ Geom plan_geom(const dcpse_plan_s* P) {
 
 int check_plan(dcpse_plan_t* P) {
     if (!P) return fail(DCPSE_ERR_ARG, "null plan");
+    t_plan_stream = P->stream;
     return DCPSE_OK;
 }
 
@@ -800,8 +946,7 @@ int surface_finish(dcpse_plan_s* P, int flags) {
     dfree(P->k_term);
     dfree(P->w64);
     dfree(P->w32);
-    if (P->r16) cudaFree(P->r16);
-    P->r16 = nullptr;
+    dfree(P->r16);
     dfree(P->r32);
     P->rowptr = rp2;
     P->cols = cols2;
@@ -827,7 +972,7 @@ int surface_finish(dcpse_plan_s* P, int flags) {
         DCPSE_CK(dalloc(&P->w32, (size_t)P->nout * nnz2 + kPad));
         DCPSE_CK(cudaMemsetAsync(P->w32, 0, sizeof(float) * ((size_t)P->nout * nnz2 + kPad), s));
         if (flags & DCPSE_STORE_OUT_F32_RESID) {
-            DCPSE_CK(cudaMalloc(&P->r16, ((size_t)P->nout * nnz2 + kPad) * 2));
+            DCPSE_CK(dalloc_bytes(&P->r16, ((size_t)P->nout * nnz2 + kPad) * 2));
             DCPSE_CK(cudaMemsetAsync(P->r16, 0, ((size_t)P->nout * nnz2 + kPad) * 2, s));
         }
         if (flags & DCPSE_STORE_OUT_F32_CORR) DCPSE_CK(dalloc(&P->r32, (size_t)P->nout * nnz2 + kPad));
@@ -849,6 +994,7 @@ int dcpse_plan_create(dcpse_plan_t** plan, int dim, int n_outputs, const int* te
                       const unsigned* signatures, unsigned order, double h_over_eps) {
     if (!plan) return fail(DCPSE_ERR_ARG, "plan is NULL");
     *plan = nullptr;
+    t_plan_stream = nullptr;
     if (dim < 1 || dim > 3) return fail(DCPSE_ERR_ARG, "dim must be 1, 2 or 3");
     if (n_outputs < 1 || n_outputs > kMaxOutputs) return fail(DCPSE_ERR_CAPACITY, "1..8 outputs per plan");
     if (!terms_per_output || !signatures) return fail(DCPSE_ERR_ARG, "NULL terms/signatures");
@@ -1174,29 +1320,31 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
     if (e == cudaSuccess) e = dalloc(&P->cols, nnz + kPad);
     if (e == cudaSuccess) e = fill_neighbors(a, P->rowptr, tmp, P->cols, hk, s);
     P->tstop(DCPSE_K_NEIGHBORS);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    int32_t *key = nullptr, *zord = nullptr;
+    int64_t* ztmp = nullptr;
+    cudaError_t ez = cudaErrorMemoryAllocation;
     if (e == cudaSuccess && !other_support) {
         // the particles' renumbering order (one set; P->reorder_order): the
         // apply's sliced layout may renumber rows and columns by it (the
         // cells' own order, if the order's work space cannot be had)
-        int32_t *key = nullptr, *zord = nullptr;
-        int64_t* ztmp = nullptr;
-        cudaError_t ez = dalloc(&key, (size_t)std::max<int64_t>(ns, 1));
+        ez = dalloc(&key, (size_t)std::max<int64_t>(ns, 1));
         if (ez == cudaSuccess) ez = dalloc(&zord, (size_t)std::max<int64_t>(ns, 1));
         if (ez == cudaSuccess) ez = dalloc(&ztmp, (size_t)order_tmp_elems(dim, ns, cg, P->reorder_order));
         if (ez == cudaSuccess) ez = particle_order(dim, ps, ns, cg, P->reorder_order, key, ztmp, zord, s);
-        if (ez == cudaSuccess) ez = cudaStreamSynchronize(s);
-        dfree(key);
-        dfree(ztmp);
+        if (ez != cudaSuccess) cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    dfree(key);
+    dfree(ztmp);
+    if (e == cudaSuccess && !other_support) {
         if (ez == cudaSuccess) {
-            P->cell_order = zord;
+            std::swap(P->cell_order, zord);
         } else {
-            dfree(zord);
-            cudaGetLastError();
             P->cell_order = cidx;
             cidx = nullptr;
         }
     }
+    dfree(zord);
     cleanup();
     if (e != cudaSuccess) return fail(DCPSE_ERR_CUDA, std::string("neighbour build: ") + cudaGetErrorString(e));
     P->nnz = nnz;
@@ -1222,36 +1370,33 @@ int dcpse_set_neighbors(dcpse_plan_t* P, int64_t n, int64_t nnz, const int64_t* 
     DCPSE_CK(dalloc(&P->cols, nnz + kPad));
     DCPSE_CK(cudaMemcpyAsync(P->rowptr, d_rowptr, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToDevice, s));
     if (nnz > 0) DCPSE_CK(cudaMemcpyAsync(P->cols, d_cols, sizeof(int32_t) * nnz, cudaMemcpyDeviceToDevice, s));
-    {
-        unsigned long long* bad = nullptr;
-        DCPSE_CK(dalloc(&bad, 1));
-        DCPSE_CK(cudaMemsetAsync(bad, 0, sizeof(unsigned long long), s));
-        int64_t work = std::max<int64_t>(n, nnz);
+    // violations and the longest row, in one pass and one copy
+    unsigned long long* chk = nullptr;
+    DCPSE_CK(dalloc(&chk, 2));
+    unsigned long long h[2] = {0, 0};
+    const int64_t work = std::max<int64_t>(n, nnz);
+    cudaError_t e = cudaMemsetAsync(chk, 0, sizeof h, s);
+    if (e == cudaSuccess) {
         csr_check_kernel<<<std::max(1, (int)std::min<int64_t>(num_sms() * 8, (work + 255) / 256)), 256, 0, s>>>(
-            P->rowptr, P->cols, n, nnz, P->two_set() ? P->n_sup : n, bad);
-        unsigned long long hb = 0;
-        cudaError_t e = cudaMemcpyAsync(&hb, bad, sizeof hb, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        dfree(bad);
-        DCPSE_CK(e);
-        if (hb != 0) {
-            dfree(P->rowptr);
-            P->list_version++;
-            dfree(P->cols);
-            P->n = -1;
-            P->nnz = 0;
-            return fail(DCPSE_ERR_ARG, "invalid CSR neighbour list (row offsets or column indices)");
-        }
+            P->rowptr, P->cols, n, nnz, P->two_set() ? P->n_sup : n, chk);
+        if (n > 0)
+            row_max_kernel<<<std::max(1, std::min(num_sms() * 4, (int)((n + 255) / 256))), 256, 0, s>>>(
+                P->rowptr, n, reinterpret_cast<int*>(chk + 1));
+        e = cudaGetLastError();
     }
-    int* mk = nullptr;
-    DCPSE_CK(dalloc(&mk, 1));
-    DCPSE_CK(cudaMemsetAsync(mk, 0, sizeof(int), s));
-    if (n > 0) row_max_kernel<<<std::max(1, std::min(num_sms() * 4, (int)((n + 255) / 256))), 256, 0, s>>>(P->rowptr, n, mk);
-    int hk = 0;
-    DCPSE_CK(cudaMemcpyAsync(&hk, mk, sizeof(int), cudaMemcpyDeviceToHost, s));
-    DCPSE_CK(cudaStreamSynchronize(s));
-    dfree(mk);
-    P->maxk = hk;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, chk, sizeof h, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    dfree(chk);
+    DCPSE_CK(e);
+    if (h[0] != 0) {
+        dfree(P->rowptr);
+        P->list_version++;
+        dfree(P->cols);
+        P->n = -1;
+        P->nnz = 0;
+        return fail(DCPSE_ERR_ARG, "invalid CSR neighbour list (row offsets or column indices)");
+    }
+    P->maxk = (int)(h[1] & 0xffffffffu);
     return DCPSE_OK;
 }
 
@@ -1329,11 +1474,8 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
     if ((flags & DCPSE_STORE_OUT_F32) && !P->w32) DCPSE_CK(dalloc(&P->w32, (size_t)P->nout * nnz + kPad));
     if (!(flags & DCPSE_STORE_OUT_F32)) dfree(P->w32);
     if ((flags & DCPSE_STORE_OUT_F32_RESID) && !P->r16)
-        DCPSE_CK(cudaMalloc(&P->r16, ((size_t)P->nout * nnz + kPad) * 2));
-    if (!(flags & DCPSE_STORE_OUT_F32_RESID) && P->r16) {
-        cudaFree(P->r16);
-        P->r16 = nullptr;
-    }
+        DCPSE_CK(dalloc_bytes(&P->r16, ((size_t)P->nout * nnz + kPad) * 2));
+    if (!(flags & DCPSE_STORE_OUT_F32_RESID)) dfree(P->r16);
     if ((flags & DCPSE_STORE_OUT_F32_CORR) && !P->r32) DCPSE_CK(dalloc(&P->r32, (size_t)P->nout * nnz + kPad));
     if (!(flags & DCPSE_STORE_OUT_F32_CORR)) dfree(P->r32);
     AsmArgs a{};
@@ -1496,8 +1638,7 @@ int dcpse_set_term_kernels(dcpse_plan_t* P, int term, const double* d_kernels, c
     P->free_sell();
     dfree(P->w64);
     dfree(P->w32);
-    if (P->r16) cudaFree(P->r16);
-    P->r16 = nullptr;
+    dfree(P->r16);
     P->flags &= ~(DCPSE_STORE_OUT_F64 | DCPSE_STORE_OUT_F32 | DCPSE_STORE_OUT_F32_RESID);
     dfree(P->rowsum);
     P->rowsum_prec = -1;
@@ -2155,17 +2296,14 @@ int ensure_sell_resid(dcpse_plan_t* P) {
                 std::swap(P->sell_r, P->spare_r);
                 return cudaSuccess;
             }
-            return cudaMalloc(&P->sell_r, ((size_t)P->nout * P->sell_total + kPad) * 2);
+            return dalloc_bytes(&P->sell_r, ((size_t)P->nout * P->sell_total + kPad) * 2);
         },
         [&] {
             return sell_fill(P->rowptr, P->cols, nullptr, P->r16, P->nnz, P->nout, P->n, P->two_set() ? 0 : 1,
                              P->sell_row, P->sell_off, P->sell_total, nullptr, nullptr, P->sell_r, P->stream,
                              P->sell_perm);
         },
-        [&] {
-            if (P->sell_r) cudaFree(P->sell_r);
-            P->sell_r = nullptr;
-        });
+        [&] { dfree(P->sell_r); });
 }
 
 // The FP32 residual streams on the sliced layout (the second float of each
