@@ -164,6 +164,9 @@ __global__ void row_max_kernel(const int64_t* rowptr, int64_t n, int* maxk) {
 // last used one.
 constexpr int64_t kPad = 8;
 
+// Most bytes of the neighbour search's staging rows.
+constexpr int64_t kStageBytes = int64_t(2) << 30;
+
 // Largest scratch of one assembly batch; larger clouds are assembled in
 // batches of particles (the result does not depend on the batch size).
 constexpr int64_t kAsmScratchBytes = int64_t(512) << 20;
@@ -1282,7 +1285,7 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
     if (e == cudaSuccess) e = dalloc(&maxk, 1);
     if (e == cudaSuccess) e = cudaMemsetAsync(maxk, 0, sizeof(int), s);
     P->tstart(DCPSE_K_NEIGHBORS);
-    if (e == cudaSuccess) e = build_cells(dim, ps, ns, cg, cell, ccount, cstart, fill, cidx, spos, srel, scan_tmp, s);
+    if (e == cudaSuccess) e = build_cells(dim, ps, ns, cg, plan_geom(P), cell, ccount, cstart, fill, cidx, spos, srel, scan_tmp, s);
     NbrArgs a{};
     a.dim = dim;
     a.pd = d_pos;
@@ -1309,16 +1312,35 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
         for (int d = 0; d < dim; ++d)
             if (P->per[d] && cg.nc[d] < 3) a.fast = 0;
     }
-    if (e == cudaSuccess) e = count_neighbors(a, counts, maxk, s);
+    // one search for counts and columns, into staging rows of 1.3 times the
+    // cutoff ball's mean occupancy + 16 entries (a jittered lattice's longest row
+    // is 1.2 times the mean), when they take at most kStageBytes
+    int row_cap = 0;
+    if (!other_support && stage_neighbors_serves(a)) {
+        double ball = dim == 2 ? 3.14159265 * rmax * rmax : 4.18879020 * rmax * rmax * rmax;
+        for (int d = 0; d < dim; ++d) ball /= std::max(hi[d] - lo[d], rmax);
+        const double want = std::min(1.3 * ball * (double)n + 16.0, 1024.0);
+        row_cap = ((int)want + 31) / 32 * 32;
+        if ((int64_t)row_cap * n * (int64_t)sizeof(int32_t) > kStageBytes || dalloc(&tmp, (size_t)row_cap * n) != cudaSuccess) {
+            cudaGetLastError();
+            row_cap = 0;
+        }
+    }
+    if (e == cudaSuccess) e = row_cap > 0 ? stage_neighbors(a, counts, maxk, tmp, row_cap, s) : count_neighbors(a, counts, maxk, s);
     if (e == cudaSuccess) e = exclusive_scan_i32(counts, n, P->rowptr, scan_tmp, s);
     int64_t nnz = 0;
     int hk = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&nnz, P->rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&hk, maxk, sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess) e = dalloc(&tmp, nnz);
+    if (hk > row_cap) {  // (no staging rows, or a row longer than them)
+        dfree(tmp);
+        row_cap = 0;
+    }
+    if (e == cudaSuccess && row_cap == 0) e = dalloc(&tmp, nnz);
     if (e == cudaSuccess) e = dalloc(&P->cols, nnz + kPad);
-    if (e == cudaSuccess) e = fill_neighbors(a, P->rowptr, tmp, P->cols, hk, s);
+    if (e == cudaSuccess)
+        e = row_cap > 0 ? sort_staged(a, P->rowptr, tmp, row_cap, P->cols, s) : fill_neighbors(a, P->rowptr, tmp, P->cols, s);
     P->tstop(DCPSE_K_NEIGHBORS);
     int32_t *key = nullptr, *zord = nullptr;
     int64_t* ztmp = nullptr;

@@ -43,7 +43,7 @@ constexpr int kOrderKeyBits = 23;
 int64_t order_tmp_elems(int dim, int64_t n, const CellGrid& g, int mode);
 cudaError_t particle_order(int dim, const double* pos, int64_t n, const CellGrid& g, int mode, int32_t* key,
                            int64_t* tmp, int32_t* order, cudaStream_t s);
-cudaError_t build_cells(int dim, const double* pos, int64_t n, const CellGrid& g, int32_t* d_cell,
+cudaError_t build_cells(int dim, const double* pos, int64_t n, const CellGrid& g, const Geom& geom, int32_t* d_cell,
                         int32_t* d_ccount, int64_t* d_cstart, int64_t* d_fill, int32_t* d_cidx, double* d_spos,
                         float4* d_srel, int64_t* d_scan_tmp, cudaStream_t s);
 
@@ -69,9 +69,15 @@ struct NbrArgs {
 // Count pass: counts[p] = number of neighbours; also atomically maxes *d_maxk.
 cudaError_t count_neighbors(const NbrArgs& a, int32_t* counts, int* d_maxk, cudaStream_t s);
 // Fill pass: unsorted neighbours of p into tmp[rowptr[p] ...], then sorted
-// ascending into cols (maxk: the longest row, from the count pass).
-cudaError_t fill_neighbors(const NbrArgs& a, const int64_t* rowptr, int32_t* tmp, int32_t* cols, int maxk,
-                           cudaStream_t s);
+// ascending into cols.
+cudaError_t fill_neighbors(const NbrArgs& a, const int64_t* rowptr, int32_t* tmp, int32_t* cols, cudaStream_t s);
+// One search for counts and columns (one set on a packed grid, the domain set
+// being the support set): the neighbours of p, unsorted, to stage[p * cap ...],
+// the first cap of them; then sorted into cols, when no row is longer than cap.
+bool stage_neighbors_serves(const NbrArgs& a);
+cudaError_t stage_neighbors(const NbrArgs& a, int32_t* counts, int* d_maxk, int32_t* stage, int cap, cudaStream_t s);
+cudaError_t sort_staged(const NbrArgs& a, const int64_t* rowptr, const int32_t* stage, int cap, int32_t* cols,
+                        cudaStream_t s);
 
 // --------------------------------------------------------------- assembly --
 // Tables describing the bases of a plan, resident on the device.

@@ -21,6 +21,7 @@
 // FP64 predicate itself, as are particles outside the grid, NaN positions
 // and periodic axes with fewer than three cells.  The lists are the same bit
 // for bit.
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cstring>
@@ -171,7 +172,7 @@ __global__ void cell_id_kernel(int dim, const double* __restrict__ pos, int64_t 
 }
 
 __global__ void cell_fill_kernel(int dim, const double* __restrict__ pos, int64_t n, const int32_t* __restrict__ cell,
-                                 CellGrid g, int64_t* fill, int32_t* __restrict__ cidx, double* __restrict__ spos,
+                                 CellGrid g, Geom geom, int64_t* fill, int32_t* __restrict__ cidx, double* __restrict__ spos,
                                  float4* __restrict__ srel) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         unsigned long long slot = atomicAdd((unsigned long long*)&fill[cell[i]], 1ull);
@@ -182,11 +183,15 @@ __global__ void cell_fill_kernel(int dim, const double* __restrict__ pos, int64_
             const double x = pos[i * dim + d];
             spos[slot * dim + d] = x;
             // offset from the cell's lower corner; NaN (always the FP64
-            // test) for a particle clamped into an edge cell
+            // test) for a particle clamped into an edge cell, along a
+            // periodic axis for any outside the box (whose stencil is still
+            // its edge cell's, see nbr_group_kernel)
             const int c = cell_coord(x, g.lo[d], g.cs[d], g.nc[d]);
             if (d == 0) cx = c;
             const double rel = x - (g.lo[d] + (double)c * g.cs[d]);
-            r[d] = (rel >= -0.5 * g.cs[d] && rel <= 1.5 * g.cs[d]) ? (float)rel : __int_as_float(0x7fc00000);
+            const double slack = geom.per[d] ? 1e-6 : 0.5;
+            r[d] = (rel >= -slack * g.cs[d] && rel <= (1.0 + slack) * g.cs[d]) ? (float)rel
+                                                                            : __int_as_float(0x7fc00000);
         }
         // w: the cell's index along axis 0, for candidates taken from a run
         // of cells along that axis
@@ -597,88 +602,85 @@ __global__ void __launch_bounds__(256) nbr_packed_kernel(NbrArgs a, int32_t* __r
     }
 }
 
-// Warp per row: rank of each entry among the row's entries -> sorted output.
-__global__ void __launch_bounds__(256) sort_rows_kernel(int64_t n, const int64_t* __restrict__ rowptr,
-                                                        const int32_t* __restrict__ tmp, int32_t* __restrict__ cols) {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t p = warp0; p < n; p += nwarps) {
-        int64_t b = rowptr[p], e = rowptr[p + 1];
-        int k = (int)(e - b);
-        for (int i0 = 0; i0 < k; i0 += 32) {
-            int i = i0 + lane;
-            int32_t v = (i < k) ? tmp[b + i] : 0;
-            int rank = 0;
-            for (int j = 0; j < k; ++j) rank += (tmp[b + j] < v);
-            if (i < k) cols[b + rank] = v;
+#include "dcpse_nbr_group.cuh"
+
+// A row's entries in the registers of a warp (lane l holds entries l KPL .. l KPL
+// + KPL - 1), sorted by a bitonic network (partners KPL or more apart are
+// exchanged by shuffles).
+template <int KPL>
+__device__ __forceinline__ void sort_row(const int32_t* __restrict__ src, int k, int lane, int32_t* __restrict__ dst) {
+    constexpr int N = 32 * KPL;
+    int32_t v[KPL];
+#pragma unroll
+    for (int s = 0; s < KPL; ++s) {
+        const int e = lane * KPL + s;
+        v[s] = e < k ? src[e] : INT32_MAX;
+    }
+#pragma unroll
+    for (int size = 2; size <= N; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride < KPL) {
+#pragma unroll
+                for (int s = 0; s < KPL; ++s) {
+                    const int s2 = s ^ stride;
+                    if (s2 > s) {
+                        const bool asc = ((lane * KPL + s) & size) == 0;
+                        const int32_t x = v[s], y = v[s2];
+                        if ((x > y) == asc) {
+                            v[s] = y;
+                            v[s2] = x;
+                        }
+                    }
+                }
+            } else {
+                const int ls = stride / KPL;
+                const bool lower = (lane & ls) == 0;
+#pragma unroll
+                for (int s = 0; s < KPL; ++s) {
+                    const int32_t o = __shfl_xor_sync(0xffffffffu, v[s], ls);
+                    const bool asc = ((lane * KPL + s) & size) == 0;
+                    v[s] = (lower == asc) ? min(v[s], o) : max(v[s], o);
+                }
+            }
         }
+    }
+#pragma unroll
+    for (int s = 0; s < KPL; ++s) {
+        const int e = lane * KPL + s;
+        if (e < k) dst[e] = v[s];
     }
 }
 
-// Warp per row, rows of up to 32 KPL entries: a bitonic sort in registers
-// (lane l holds entries l KPL .. l KPL + KPL - 1; partners KPL or more apart
-// are exchanged by shuffles).  Longer rows take the rank sort above.
-template <int KPL>
-__global__ void __launch_bounds__(256) sort_rows_bitonic_kernel(int64_t n, const int64_t* __restrict__ rowptr,
-                                                                const int32_t* __restrict__ tmp,
-                                                                int32_t* __restrict__ cols) {
-    constexpr int N = 32 * KPL;
+// Warp per row: its entries, from tmp at the row's own offset or (cap > 0) from
+// its staging row of cap entries, sorted into cols.  The network is the smallest
+// that holds the row (32, 64, 128 or 256 entries); longer rows rank every entry.
+__global__ void __launch_bounds__(256) sort_rows_kernel(int64_t n, const int64_t* __restrict__ rowptr,
+                                                        const int32_t* __restrict__ tmp, int cap,
+                                                        int32_t* __restrict__ cols) {
     const int lane = threadIdx.x & 31;
     const int64_t warp0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t p = warp0; p < n; p += nwarps) {
         const int64_t b = rowptr[p];
         const int k = (int)(rowptr[p + 1] - b);
-        if (k > N) {
+        const int32_t* src = tmp + (cap > 0 ? p * cap : b);
+        if (k <= 32) {
+            sort_row<1>(src, k, lane, cols + b);
+        } else if (k <= 64) {
+            sort_row<2>(src, k, lane, cols + b);
+        } else if (k <= 128) {
+            sort_row<4>(src, k, lane, cols + b);
+        } else if (k <= 256) {
+            sort_row<8>(src, k, lane, cols + b);
+        } else {
             for (int i0 = 0; i0 < k; i0 += 32) {
                 const int i = i0 + lane;
-                const int32_t v = (i < k) ? tmp[b + i] : 0;
+                const int32_t v = (i < k) ? src[i] : 0;
                 int rank = 0;
-                for (int j = 0; j < k; ++j) rank += (tmp[b + j] < v);
+                for (int j = 0; j < k; ++j) rank += (src[j] < v);
                 if (i < k) cols[b + rank] = v;
             }
-            continue;
-        }
-        int32_t v[KPL];
-#pragma unroll
-        for (int s = 0; s < KPL; ++s) {
-            const int e = lane * KPL + s;
-            v[s] = e < k ? tmp[b + e] : INT32_MAX;
-        }
-#pragma unroll
-        for (int size = 2; size <= N; size <<= 1) {
-#pragma unroll
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                if (stride < KPL) {
-#pragma unroll
-                    for (int s = 0; s < KPL; ++s) {
-                        const int s2 = s ^ stride;
-                        if (s2 > s) {
-                            const bool asc = ((lane * KPL + s) & size) == 0;
-                            const int32_t x = v[s], y = v[s2];
-                            if ((x > y) == asc) {
-                                v[s] = y;
-                                v[s2] = x;
-                            }
-                        }
-                    }
-                } else {
-                    const int ls = stride / KPL;
-                    const bool lower = (lane & ls) == 0;
-#pragma unroll
-                    for (int s = 0; s < KPL; ++s) {
-                        const int32_t o = __shfl_xor_sync(0xffffffffu, v[s], ls);
-                        const bool asc = ((lane * KPL + s) & size) == 0;
-                        v[s] = (lower == asc) ? min(v[s], o) : max(v[s], o);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int s = 0; s < KPL; ++s) {
-            const int e = lane * KPL + s;
-            if (e < k) cols[b + e] = v[s];
         }
     }
 }
@@ -748,7 +750,7 @@ cudaError_t bounding_box(int dim, const double* a, int64_t na, const double* b, 
     return cudaGetLastError();
 }
 
-cudaError_t build_cells(int dim, const double* pos, int64_t n, const CellGrid& g, int32_t* d_cell, int32_t* d_ccount,
+cudaError_t build_cells(int dim, const double* pos, int64_t n, const CellGrid& g, const Geom& geom, int32_t* d_cell, int32_t* d_ccount,
                         int64_t* d_cstart, int64_t* d_fill, int32_t* d_cidx, double* d_spos, float4* d_srel,
                         int64_t* d_scan_tmp, cudaStream_t s) {
     int64_t ncell = (int64_t)g.nc[0] * g.nc[1] * g.nc[2];
@@ -760,7 +762,7 @@ cudaError_t build_cells(int dim, const double* pos, int64_t n, const CellGrid& g
     e = cudaMemcpyAsync(d_fill, d_cstart, sizeof(int64_t) * ncell, cudaMemcpyDeviceToDevice, s);
     if (e != cudaSuccess) return e;
     if (n > 0)
-        cell_fill_kernel<<<grid_for(n, 256), 256, 0, s>>>(dim, pos, n, d_cell, g, d_fill, d_cidx, d_spos, d_srel);
+        cell_fill_kernel<<<grid_for(n, 256), 256, 0, s>>>(dim, pos, n, d_cell, g, geom, d_fill, d_cidx, d_spos, d_srel);
     return cudaGetLastError();
 }
 
@@ -877,8 +879,27 @@ cudaError_t count_neighbors(const NbrArgs& a, int32_t* counts, int* d_maxk, cuda
     return cudaGetLastError();
 }
 
-cudaError_t fill_neighbors(const NbrArgs& a, const int64_t* rowptr, int32_t* tmp, int32_t* cols, int maxk,
-                           cudaStream_t s) {
+bool stage_neighbors_serves(const NbrArgs& a) { return group_side(a) > 0; }
+
+cudaError_t stage_neighbors(const NbrArgs& a, int32_t* counts, int* d_maxk, int32_t* stage, int cap, cudaStream_t s) {
+    if (a.n_dom == 0) return cudaSuccess;
+    const int G = group_side(a);
+    if (a.dim == 3)
+        return G == 2 ? launch_group<3, 2, 4>(a, counts, d_maxk, stage, cap, s)
+                      : launch_group<3, 1, 4>(a, counts, d_maxk, stage, cap, s);
+    if (G == 4) return launch_group<2, 4, 2>(a, counts, d_maxk, stage, cap, s);
+    return G == 2 ? launch_group<2, 2, 2>(a, counts, d_maxk, stage, cap, s)
+                  : launch_group<2, 1, 2>(a, counts, d_maxk, stage, cap, s);
+}
+
+cudaError_t sort_staged(const NbrArgs& a, const int64_t* rowptr, const int32_t* stage, int cap, int32_t* cols,
+                        cudaStream_t s) {
+    if (a.n_dom == 0) return cudaSuccess;
+    sort_rows_kernel<<<grid_for(a.n_dom * 32, 256), 256, 0, s>>>(a.n_dom, rowptr, stage, cap, cols);
+    return cudaGetLastError();
+}
+
+cudaError_t fill_neighbors(const NbrArgs& a, const int64_t* rowptr, int32_t* tmp, int32_t* cols, cudaStream_t s) {
     if (a.n_dom == 0) return cudaSuccess;
     int grid = grid_for(a.n_dom * 32, 256);
     if (a.packed) {
@@ -892,12 +913,7 @@ cudaError_t fill_neighbors(const NbrArgs& a, const int64_t* rowptr, int32_t* tmp
     } else {
         nbr_kernel<3, true><<<grid, 256, 0, s>>>(a, nullptr, nullptr, rowptr, tmp);
     }
-    if (maxk <= 128)
-        sort_rows_bitonic_kernel<4><<<grid, 256, 0, s>>>(a.n_dom, rowptr, tmp, cols);
-    else if (maxk <= 256)
-        sort_rows_bitonic_kernel<8><<<grid, 256, 0, s>>>(a.n_dom, rowptr, tmp, cols);
-    else
-        sort_rows_kernel<<<grid, 256, 0, s>>>(a.n_dom, rowptr, tmp, cols);
+    sort_rows_kernel<<<grid, 256, 0, s>>>(a.n_dom, rowptr, tmp, 0, cols);
     return cudaGetLastError();
 }
 
