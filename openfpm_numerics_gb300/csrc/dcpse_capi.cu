@@ -1238,6 +1238,7 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
                     g.cs[d] = 1.0;
                     g.lo[d] = 0.0;
                 }
+                g.ics[d] = 1.0 / g.cs[d];
                 total *= g.nc[d];
             }
             if (total <= cap) break;
@@ -1352,7 +1353,7 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
         ez = dalloc(&key, (size_t)std::max<int64_t>(ns, 1));
         if (ez == cudaSuccess) ez = dalloc(&zord, (size_t)std::max<int64_t>(ns, 1));
         if (ez == cudaSuccess) ez = dalloc(&ztmp, (size_t)order_tmp_elems(dim, ns, cg, P->reorder_order));
-        if (ez == cudaSuccess) ez = particle_order(dim, ps, ns, cg, P->reorder_order, key, ztmp, zord, s);
+        if (ez == cudaSuccess) ez = particle_order(dim, ps, cell, ns, cg, P->reorder_order, key, ztmp, zord, s);
         if (ez != cudaSuccess) cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

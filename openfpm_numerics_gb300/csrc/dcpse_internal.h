@@ -16,7 +16,7 @@ namespace dcpse {
 // ------------------------------------------------------------ neighbours --
 struct CellGrid {
     double lo[kMaxDim];
-    double cs[kMaxDim];
+    double cs[kMaxDim], ics[kMaxDim];  // side and its reciprocal
     int nc[kMaxDim];
 };
 
@@ -41,7 +41,8 @@ cudaError_t bounding_box(int dim, const double* a, int64_t na, const double* b, 
 // tmp: order_tmp_elems() int64; key: n int32.
 constexpr int kOrderKeyBits = 23;
 int64_t order_tmp_elems(int dim, int64_t n, const CellGrid& g, int mode);
-cudaError_t particle_order(int dim, const double* pos, int64_t n, const CellGrid& g, int mode, int32_t* key,
+cudaError_t particle_order(int dim, const double* pos, const int32_t* cell, int64_t n, const CellGrid& g, int mode,
+                           int32_t* key,
                            int64_t* tmp, int32_t* order, cudaStream_t s);
 cudaError_t build_cells(int dim, const double* pos, int64_t n, const CellGrid& g, const Geom& geom, int32_t* d_cell,
                         int32_t* d_ccount, int64_t* d_cstart, int64_t* d_fill, int32_t* d_cidx, double* d_spos,

@@ -201,8 +201,8 @@ __global__ void __launch_bounds__(256) nbr_group_kernel(NbrArgs a, GroupGrid gg,
                                     const double xp = a.pd[(int64_t)pi * DIM + d], xq = a.spos[(int64_t)t[u] * DIM + d];
                                     o[d] = offset1(a.geom, d, xp, xq);
                                     const int nc = a.cells.nc[d];
-                                    int dc = abs(cell_coord(xp, a.cells.lo[d], a.cells.cs[d], nc) -
-                                                 cell_coord(xq, a.cells.lo[d], a.cells.cs[d], nc));
+                                    int dc = abs(cell_coord(xp, a.cells.lo[d], a.cells.ics[d], nc) -
+                                                 cell_coord(xq, a.cells.lo[d], a.cells.ics[d], nc));
                                     if (a.geom.per[d]) dc = min(dc, nc - dc);
                                     near = near && dc <= kPackR;
                                 }

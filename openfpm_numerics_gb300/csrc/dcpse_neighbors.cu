@@ -117,6 +117,31 @@ __global__ void scan_tiles(const int32_t* __restrict__ in, int64_t n, const int6
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = tile_off[gridDim.x];
 }
 
+// Small inputs: one block walks the tiles (one launch instead of three, each of
+// which takes about as long as a tile does here).
+constexpr int64_t kScanOneBlock = 4;
+__global__ void __launch_bounds__(kScanThreads) scan_one_block(const int32_t* __restrict__ in, int64_t n,
+                                                               int64_t* __restrict__ out) {
+    int64_t carry = 0;
+    for (int64_t t0 = 0; t0 < n; t0 += kScanTile) {
+        const int64_t base = t0 + (int64_t)threadIdx.x * kScanItems;
+        int64_t v[kScanItems], s = 0, tot;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            v[i] = (base + i < n) ? (int64_t)in[base + i] : 0;
+            s += v[i];
+        }
+        int64_t ex = block_excl_scan(s, &tot) + carry;
+#pragma unroll
+        for (int i = 0; i < kScanItems; ++i) {
+            if (base + i < n) out[base + i] = ex;
+            ex += v[i];
+        }
+        carry += tot;
+    }
+    if (threadIdx.x == 0) out[n] = carry;
+}
+
 __device__ __forceinline__ unsigned long long ord_of(double x) {
     unsigned long long u = (unsigned long long)__double_as_longlong(x);
     return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
@@ -129,42 +154,58 @@ double from_ord(unsigned long long u) {
     return d;
 }
 
-__global__ void bbox_kernel(int dim, const double* __restrict__ p, int64_t n, unsigned long long* mm) {
-    double lo[kMaxDim], hi[kMaxDim];
+// (ordered bits compared as integers: FP64 minima and maxima held the FP64 pipe;
+// NaN is passed over, as by fmin and fmax)
+__global__ void __launch_bounds__(256) bbox_kernel(int dim, const double* __restrict__ p, int64_t n,
+                                                   unsigned long long* mm) {
+    unsigned long long lo[kMaxDim], hi[kMaxDim];
     for (int d = 0; d < kMaxDim; ++d) {
-        lo[d] = INFINITY;
-        hi[d] = -INFINITY;
+        lo[d] = ~0ull;
+        hi[d] = 0ull;
     }
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        for (int d = 0; d < dim; ++d) {
-            double x = p[i * dim + d];
-            lo[d] = fmin(lo[d], x);
-            hi[d] = fmax(hi[d], x);
+#pragma unroll
+        for (int d = 0; d < kMaxDim; ++d) {
+            if (d >= dim) break;
+            const double x = p[i * dim + d];
+            const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+            if (h > 0x7ff00000u || (h == 0x7ff00000u && __double2loint(x) != 0)) continue;
+            const unsigned long long u = ord_of(x);
+            lo[d] = min(lo[d], u);
+            hi[d] = max(hi[d], u);
         }
     for (int d = 0; d < dim; ++d) {
         for (int o = 16; o > 0; o >>= 1) {
-            lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-            hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+            lo[d] = min(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+            hi[d] = max(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
         }
         if ((threadIdx.x & 31) == 0) {
-            atomicMin(&mm[d], ord_of(lo[d]));
-            atomicMax(&mm[kMaxDim + d], ord_of(hi[d]));
+            if (lo[d] != ~0ull) atomicMin(&mm[d], lo[d]);
+            if (hi[d] != 0ull) atomicMax(&mm[kMaxDim + d], hi[d]);
         }
     }
 }
 
-__device__ __forceinline__ int cell_coord(double x, double lo, double cs, int nc) {
-    double v = floor((x - lo) / cs);
-    if (!(v >= 0.0)) return 0;  // also catches NaN
-    if (v >= (double)nc) return nc - 1;
-    return (int)v;
+// cell of x along an axis, clamped into the grid (NaN: an edge cell); ics = 1 / cs.
+// Three FP64 instructions: the pipe bounds the kernels that bin particles (a
+// division and comparisons made it 13).
+__device__ __forceinline__ int cell_coord(double x, double lo, double ics, int nc) {
+    return min(max(__double2int_rd((x - lo) * ics), 0), nc - 1);
+}
+
+// coordinates of linear cell index `lin`
+__device__ __forceinline__ void cell_of(int lin, const CellGrid& g, int (&c)[kMaxDim]) {
+    const int row = lin / g.nc[0];
+    c[0] = lin - row * g.nc[0];
+    c[2] = row / g.nc[1];
+    c[1] = row - c[2] * g.nc[1];
 }
 
 __global__ void cell_id_kernel(int dim, const double* __restrict__ pos, int64_t n, CellGrid g,
                                int32_t* __restrict__ cell, int32_t* __restrict__ ccount) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         int c[kMaxDim] = {0, 0, 0};
-        for (int d = 0; d < dim; ++d) c[d] = cell_coord(pos[i * dim + d], g.lo[d], g.cs[d], g.nc[d]);
+        for (int d = 0; d < dim; ++d) c[d] = cell_coord(pos[i * dim + d], g.lo[d], g.ics[d], g.nc[d]);
         int lin = c[0] + g.nc[0] * (c[1] + g.nc[1] * c[2]);
         cell[i] = lin;
         atomicAdd(&ccount[lin], 1);
@@ -178,7 +219,9 @@ __global__ void cell_fill_kernel(int dim, const double* __restrict__ pos, int64_
         unsigned long long slot = atomicAdd((unsigned long long*)&fill[cell[i]], 1ull);
         cidx[slot] = (int32_t)i;
         float r[kMaxDim] = {0.f, 0.f, 0.f};
-        int cx = 0;
+        int cc[kMaxDim];
+        cell_of(cell[i], g, cc);
+        const int cx = cc[0];
         for (int d = 0; d < dim; ++d) {
             const double x = pos[i * dim + d];
             spos[slot * dim + d] = x;
@@ -186,12 +229,9 @@ __global__ void cell_fill_kernel(int dim, const double* __restrict__ pos, int64_
             // test) for a particle clamped into an edge cell, along a
             // periodic axis for any outside the box (whose stencil is still
             // its edge cell's, see nbr_group_kernel)
-            const int c = cell_coord(x, g.lo[d], g.cs[d], g.nc[d]);
-            if (d == 0) cx = c;
-            const double rel = x - (g.lo[d] + (double)c * g.cs[d]);
-            const double slack = geom.per[d] ? 1e-6 : 0.5;
-            r[d] = (rel >= -slack * g.cs[d] && rel <= (1.0 + slack) * g.cs[d]) ? (float)rel
-                                                                            : __int_as_float(0x7fc00000);
+            const float rel = (float)fma(-(double)cc[d], g.cs[d], x - g.lo[d]), side = (float)g.cs[d];
+            const float slack = geom.per[d] ? 1e-6f : 0.5f;
+            r[d] = (rel >= -slack * side && rel <= (1.0f + slack) * side) ? rel : __int_as_float(0x7fc00000);
         }
         // w: the cell's index along axis 0, for candidates taken from a run
         // of cells along that axis
@@ -226,7 +266,7 @@ __device__ __forceinline__ void make_stencil(const NbrArgs& a, const double* xp,
             continue;
         }
         const int nc = a.cells.nc[d];
-        const int c = cell_coord(xp[d], a.cells.lo[d], a.cells.cs[d], nc);
+        const int c = cell_coord(xp[d], a.cells.lo[d], a.cells.ics[d], nc);
         S.c[d] = c;
         S.rpc[d] = (float)(xp[d] - (a.cells.lo[d] + (double)c * a.cells.cs[d]));
         int w[3];
@@ -408,7 +448,7 @@ __device__ __forceinline__ void make_pack_stencil(const NbrArgs& a, const double
             continue;
         }
         const int nc = a.cells.nc[d];
-        const int c = cell_coord(xp[d], a.cells.lo[d], a.cells.cs[d], nc);
+        const int c = cell_coord(xp[d], a.cells.lo[d], a.cells.ics[d], nc);
         S.c[d] = c;
         S.rpc[d] = (float)(xp[d] - (a.cells.lo[d] + (double)c * a.cells.cs[d]));
         if (d == 0 && a.geom.per[0] && (c - kPackR < 0 || c + kPackR >= nc)) S.xwrap = true;
@@ -721,6 +761,10 @@ cudaError_t exclusive_scan_i32(const int32_t* in, int64_t n, int64_t* out, int64
     if (ntiles == 0) {
         return cudaMemsetAsync(out, 0, sizeof(int64_t), s);
     }
+    if (ntiles <= kScanOneBlock) {
+        scan_one_block<<<1, kScanThreads, 0, s>>>(in, n, out);
+        return cudaGetLastError();
+    }
     scan_tile_sums<<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, n, tmp);
     scan_tile_offsets<<<1, kScanThreads, 0, s>>>(tmp, ntiles);
     scan_tiles<<<(unsigned)ntiles, kScanThreads, 0, s>>>(in, n, tmp, out);
@@ -778,25 +822,27 @@ struct OrderGrid {
     int nc[kMaxDim];          // row-major grid
 };
 
-__device__ __forceinline__ int32_t order_key(const double* x, int dim, const CellGrid& g, const OrderGrid& o) {
+__device__ __forceinline__ int32_t order_key(const double* x, int cell, int dim, const CellGrid& g, const OrderGrid& o) {
     int32_t k = 0;
     if (o.mode == 0) {
-        int c[kMaxDim] = {0, 0, 0};
-        for (int d = 0; d < dim; ++d) c[d] = cell_coord(x[d], g.lo[d], g.cs[d], g.nc[d]);
+        int c[kMaxDim];
+        cell_of(cell, g, c);
         for (int b = 0; b < o.bits; ++b)
             for (int d = 0; d < dim; ++d) k |= ((c[d] >> (o.shift + b)) & 1) << (b * dim + d);
     } else {
-        for (int d = dim - 1; d >= 0; --d) k = k * o.nc[d] + cell_coord(x[d], o.lo[d], o.cs[d], o.nc[d]);
+        for (int d = dim - 1; d >= 0; --d) k = k * o.nc[d] + cell_coord(x[d], o.lo[d], 1.0 / o.cs[d], o.nc[d]);
     }
     return k;
 }
 
-__global__ void order_key_kernel(int dim, const double* __restrict__ pos, int64_t n, CellGrid g, OrderGrid o,
+__global__ void order_key_kernel(int dim, const double* __restrict__ pos, const int32_t* __restrict__ cell, int64_t n,
+                                 CellGrid g, OrderGrid o,
                                  int32_t* __restrict__ key, int32_t* __restrict__ hist) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         double x[kMaxDim] = {0.0, 0.0, 0.0};
-        for (int d = 0; d < dim; ++d) x[d] = pos[i * dim + d];
-        const int32_t k = order_key(x, dim, g, o);
+        if (o.mode != 0)
+            for (int d = 0; d < dim; ++d) x[d] = pos[i * dim + d];
+        const int32_t k = order_key(x, cell[i], dim, g, o);
         key[i] = k;
         atomicAdd(&hist[k], 1);
     }
@@ -847,7 +893,8 @@ int64_t order_tmp_elems(int dim, int64_t n, const CellGrid& g, int mode) {
     return 3 * nkeys + scan_tmp_elems(nkeys) + 1;
 }
 
-cudaError_t particle_order(int dim, const double* pos, int64_t n, const CellGrid& g, int mode, int32_t* key,
+cudaError_t particle_order(int dim, const double* pos, const int32_t* cell, int64_t n, const CellGrid& g, int mode,
+                           int32_t* key,
                            int64_t* tmp, int32_t* order, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     int64_t nkeys = 0;
@@ -857,7 +904,7 @@ cudaError_t particle_order(int dim, const double* pos, int64_t n, const CellGrid
     int64_t* scan_tmp = starts + nkeys + 1;
     cudaError_t e = cudaMemsetAsync(hist, 0, sizeof(int32_t) * nkeys, s);
     if (e != cudaSuccess) return e;
-    order_key_kernel<<<grid_for(n, 256), 256, 0, s>>>(dim, pos, n, g, o, key, hist);
+    order_key_kernel<<<grid_for(n, 256), 256, 0, s>>>(dim, pos, cell, n, g, o, key, hist);
     e = exclusive_scan_i32(hist, nkeys, starts, scan_tmp, s);
     if (e != cudaSuccess) return e;
     order_scatter_kernel<<<grid_for(n, 256), 256, 0, s>>>(key, n, starts, order);
