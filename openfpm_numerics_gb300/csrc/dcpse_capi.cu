@@ -458,6 +458,7 @@ struct dcpse_plan_s {
     void free_tsell() {
         dfree(tsell_row);
         dfree(tsell_cols);
+        free_narrow(tsell_narrow);
         dfree(tsell_off);
         dfree(tsell_w);
     }
@@ -535,6 +536,12 @@ struct dcpse_plan_s {
     int32_t* sell_row = nullptr;
     int64_t* sell_off = nullptr;
     int32_t* sell_cols = nullptr;
+    NarrowCols sell_narrow{}, tsell_narrow{};  // the columns in 16 bits (long lists; sell_narrow_cols)
+    static void free_narrow(NarrowCols& nc) {
+        dfree(nc.d);
+        dfree(nc.base);
+        dfree(nc.flag);
+    }
     float* sell_w = nullptr;
     void* sell_r = nullptr;  // bf16 residuals on the same layout (with r16)
     float* sell_r32 = nullptr;  // FP32 residuals on the same layout (with r32: the weight pairs)
@@ -572,6 +579,7 @@ struct dcpse_plan_s {
         dfree(sell_row);
         dfree(sell_off);
         dfree(sell_cols);
+        free_narrow(sell_narrow);
         sell_total = 0;
     }
     void free_assembly() {
@@ -879,6 +887,23 @@ int fixed_into_plan(dcpse_plan_t* P, const double* d_f, const int32_t* inv) {
     P->tstop(DCPSE_K_SPLIT);
     DCPSE_CK(e);
     return DCPSE_OK;
+}
+
+// 16-bit columns of a sliced layout whose streams (columns and nout FP32 weight
+// streams) exceed L2; from L2 the columns' bytes do not matter and the list may
+// be applied only once.  Without room the 32-bit columns serve alone.
+constexpr int64_t kNarrowStreamBytes = int64_t(128) << 20;
+cudaError_t narrow_columns(const int32_t* srow, const int64_t* off, const int32_t* cols, int64_t total, int64_t nslices,
+                           int nout, NarrowCols& nc, cudaStream_t s) {
+    if (total * (4 + 4 * (int64_t)nout) <= kNarrowStreamBytes) return cudaSuccess;
+    if (dalloc(&nc.d, (size_t)total + kPad) != cudaSuccess ||
+        dalloc(&nc.base, (size_t)narrow_bases(total, nslices)) != cudaSuccess ||
+        dalloc(&nc.flag, (size_t)nslices) != cudaSuccess) {
+        cudaGetLastError();
+        dcpse_plan_s::free_narrow(nc);
+        return cudaSuccess;
+    }
+    return sell_narrow(srow, off, cols, nslices, nc, s);
 }
 
 // SurfaceDcpse::accumulateAndDeleteNormalParticles on the plan's arrays: the
@@ -1918,6 +1943,7 @@ int dcpse_rk4_gs_stage(dcpse_plan_t* P, int stage, int precision, const void* Yu
                 a.srow = P->sell_row;
                 a.soff = P->sell_off;
                 a.scols = P->sell_cols;
+                a.narrow = P->sell_narrow;
                 a.sw = P->sell_w;
             }
         }
@@ -1968,6 +1994,8 @@ int dcpse_rk4_gs_adjoint_prepare(dcpse_plan_t* P, int precision) {
             if (e == cudaSuccess)
                 e = sell_fill(P->t_row, P->t_src, P->wT32, nullptr, P->nnz, 1, P->n, 1, P->tsell_row, P->tsell_off,
                               total, P->tsell_cols, P->tsell_w, nullptr, P->stream);
+            if (e == cudaSuccess)
+                e = narrow_columns(P->tsell_row, P->tsell_off, P->tsell_cols, total, ns, 1, P->tsell_narrow, P->stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(P->stream);
             if (e != cudaSuccess) {
                 P->free_tsell();
@@ -2002,7 +2030,7 @@ int dcpse_rk4_gs_adjoint_stage(dcpse_plan_t* P, int precision, const void* Yu, c
         RkAdjArgs<float> a{P->n, P->t_row, P->t_src, P->wT32, P->rs32, (const float*)Yu, (const float*)Yv,
                            (const float*)kbu, (const float*)kbv, (const float*)ybu, (const float*)ybv, (float*)accu,
                            (float*)accv, (float*)next_u, (float*)next_v, cy, cY, params[0], params[1], params[2],
-                           params[3], P->rk_pack, P->tsell_row, P->tsell_off, P->tsell_cols, P->tsell_w};
+                           params[3], P->rk_pack, P->tsell_row, P->tsell_off, P->tsell_cols, P->tsell_w, P->tsell_narrow};
         const int mode = P->apply_mode & 15;
         if (!(mode == 0 || mode == 4) || !P->tsell_w) a.srow = nullptr;  // a CSR schedule was asked for
         DCPSE_CK(rk_adjoint_stage<float>(a, lanes, P->stream));
@@ -2072,6 +2100,7 @@ int dcpse_rk4_gs_reverse_step(dcpse_plan_t* P, int precision, const void* const*
                 a.srow = P->tsell_row;
                 a.soff = P->tsell_off;
                 a.scols = P->tsell_cols;
+                a.narrow = P->tsell_narrow;
                 a.sw = P->tsell_w;
             }
             DCPSE_CK(rk_adjoint_stage<R>(a, lanes, P->stream));
@@ -2229,6 +2258,8 @@ int ensure_sell_layout(dcpse_plan_t* P) {
         e = sell_fill(P->rowptr, P->cols, nullptr, nullptr, P->nnz, P->nout, P->n, P->two_set() ? 0 : 1,
                       P->sell_row, P->sell_off, total, P->sell_cols, nullptr, nullptr, P->stream, P->sell_perm,
                       P->sell_perm ? P->sell_inv : nullptr);
+    if (e == cudaSuccess)
+        e = narrow_columns(P->sell_row, P->sell_off, P->sell_cols, total, ns, P->nout, P->sell_narrow, P->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(P->stream);
     if (e == cudaErrorMemoryAllocation) {
         // the layout does not fit: the CSR kernels serve
@@ -2428,6 +2459,7 @@ int apply_f32_rows(dcpse_plan_t* P, int precision, double* d_out, int64_t r0, in
         sa.srow = P->sell_row;
         sa.off = P->sell_off;
         sa.cols = P->sell_cols;
+        sa.narrow = P->sell_narrow;
         sa.w = P->sell_w;
         sa.r = resid ? static_cast<const __nv_bfloat16*>(P->sell_r) : nullptr;
         sa.r32 = pair ? P->sell_r32 : nullptr;
@@ -3005,6 +3037,7 @@ int dcpse_p2p(dcpse_plan_t* P, const double* d_f_support, int ncomp, double* d_o
                     sa.srow = P->sell_row;
                     sa.off = P->sell_off;
                     sa.cols = P->sell_cols;
+                    sa.narrow = P->sell_narrow;
                     sa.w = P->sell_w;
                     sa.total = P->sell_total;
                     sa.f2 = P->f2;

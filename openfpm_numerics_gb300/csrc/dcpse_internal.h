@@ -221,6 +221,21 @@ cudaError_t preload_apply_f32_direct();
 // inv[list row] = position, e.g. a cell order of the particles): its columns
 // are then positions, the field pair is read at positions, and outputs go to
 // list rows.
+// The columns of a sliced layout in 16 bits (sell_narrow): entry j of a slice's
+// lane is d = cols - base of its four entries [4 (j / 4), + 4) over the slice's
+// lanes, 0xffff for the row itself (and for lanes past the last row); slices
+// whose columns spread further than 65534 keep the 32-bit stream (flag 0).
+// base of entry j of the slice at off: base[narrow_base(off, s) + j / 4].
+struct NarrowCols {
+    uint16_t* d;            // [total], or null: no narrow columns
+    int32_t* base;          // [narrow_bases(total, nslices)]
+    unsigned char* flag;    // [nslices]
+};
+__host__ __device__ inline int64_t narrow_base(int64_t off, int64_t slice) { return off / 128 + slice; }
+inline int64_t narrow_bases(int64_t total, int64_t nslices) { return total / 128 + nslices + 1; }
+cudaError_t sell_narrow(const int32_t* srow, const int64_t* off, const int32_t* cols, int64_t nslices,
+                        const NarrowCols& nc, cudaStream_t s);
+
 struct SellArgs {
     const int32_t* perm;   // position -> list row, or null (identity)
     int64_t n;             // rows
@@ -228,6 +243,7 @@ struct SellArgs {
     const int32_t* srow;   // row of (slice, lane), -1 past the last row
     const int64_t* off;    // [nslices + 1] first entry of each slice
     const int32_t* cols;   // [total] entry-major within a slice
+    NarrowCols narrow;     // the columns in 16 bits (plain FP32 applies)
     const float* w;        // [NO][total]
     const __nv_bfloat16* r; // [NO][total] bf16 residuals of the weights, or null
     const float* r32;      // [NO][total] FP32 residuals w64 - w32 (weight pairs), or null
@@ -458,6 +474,7 @@ struct RkArgs {
     const int64_t* soff;
     const int32_t* scols;
     const float* sw;
+    NarrowCols narrow;
 };
 template <typename T>
 struct RkAdjArgs {
@@ -479,6 +496,7 @@ struct RkAdjArgs {
     const int64_t* soff;
     const int32_t* scols;
     const float* sw;
+    NarrowCols narrow;
     // fused reverse step: the row's own kbar read from the pairs (kbu, kbv
     // unused), the next kbar written as pairs to pack_out (next_u, next_v
     // unused), and acc_mode 1: acc = ybar + Ybar, 2: ybar = acc + Ybar (in

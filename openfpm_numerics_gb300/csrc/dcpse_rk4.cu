@@ -148,46 +148,97 @@ __global__ void __launch_bounds__(256) gs_stage_kernel(RkArgs<T> a) {
     }
 }
 
+// Entries of a row in flight in the sliced stage kernels, at four blocks per SM
+// (64 registers): 96^3 step 0.435 ms; 4 entries at five blocks 0.547, 12 at three
+// 0.466, 16 at two 0.535 ms.
+constexpr int kGsEntries = 8;
+
+// The columns of a slice's next U entries (j0 a multiple of 4), loaded one chunk
+// ahead of their use: from the slice's 16-bit stream (NarrowCols) with C16,
+// decoded only when used, else the 32-bit ones.
+template <bool C16, int U>
+struct SliceCols {
+    const int32_t* __restrict__ c;
+    const uint16_t* __restrict__ d;
+    const int32_t* __restrict__ base;
+    int32_t self;
+    int32_t raw[U], rb[U / 4];
+    __device__ __forceinline__ SliceCols(const int32_t* cols, const NarrowCols& nc, int64_t off, int64_t s, int lane,
+                                         int32_t row)
+        : c(cols + off + lane), d(C16 ? nc.d + off + lane : nullptr), base(C16 ? nc.base + narrow_base(off, s) : nullptr),
+          self(row) {}
+    // entries [j0, min(j0 + U, L)); the others are the row itself
+    __device__ __forceinline__ void load(int j0, int L) {
+        if constexpr (C16) {
+#pragma unroll
+            for (int u = 0; u < U; u += 4) rb[u / 4] = j0 + u < L ? base[(j0 >> 2) + (u >> 2)] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t at = (int64_t)(j0 + u) * 32;
+            if constexpr (C16)
+                raw[u] = j0 + u < L ? (int32_t)d[at] : 0xffff;
+            else
+                raw[u] = j0 + u < L ? c[at] : self;
+        }
+    }
+    __device__ __forceinline__ int32_t operator[](int u) const {
+        if constexpr (C16) return raw[u] == 0xffff ? self : rb[u / 4] + raw[u];
+        return raw[u];
+    }
+};
+
 // FP32 stage on the sliced ELL layout of the weights (slices of 32 rows
 // stored entry-major, rows sorted by length within windows of 256): a row per
 // thread, 8 gathers of (u, v) pairs in flight; entries past the slice end
 // take the row's own pair with weight 0 (an exact zero)
-__global__ void __launch_bounds__(256) gs_stage_sell_kernel(RkArgs<float> a, int64_t nwin) {
+template <bool C16>
+__device__ __forceinline__ void gs_stage_slice(const RkArgs<float>& a, int64_t s, int lane, int32_t row) {
     const float2* __restrict__ Y2 = static_cast<const float2*>(a.pack);
+    constexpr int U = kGsEntries;
+    const int64_t b = a.soff[s];
+    const int L = (int)((a.soff[s + 1] - b) / 32);
+    const float2 yp = Y2[row];
+    SliceCols<C16, U> col(a.scols, a.narrow, b, s, lane, row);
+    const float* __restrict__ w = a.sw + b + lane;
+    float lu = 0.f, lv = 0.f;
+    // columns and weights run one chunk ahead of the gathers
+    float wn[U];
+    col.load(0, L);
+#pragma unroll
+    for (int u = 0; u < U; ++u) wn[u] = u < L ? w[(int64_t)u * 32] : 0.f;
+    for (int j0 = 0; j0 < L; j0 += U) {
+        float2 y[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) y[u] = j0 + u < L ? Y2[col[u]] : yp;
+        float wq[U];
+        col.load(j0 + U, L);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            wq[u] = wn[u];
+            wn[u] = j0 + U + u < L ? w[(int64_t)(j0 + U + u) * 32] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            lu = fmaf(wq[u], y[u].x - yp.x, lu);
+            lv = fmaf(wq[u], y[u].y - yp.y, lv);
+        }
+    }
+    stage_update(a, row, yp.x, yp.y, lu, lv);
+}
+
+// Bound by HBM: per entry a 4-byte weight and the column, 2 bytes where the
+// slice has narrow columns (4 before).
+__global__ void __launch_bounds__(256, 4) gs_stage_sell_kernel(RkArgs<float> a, int64_t nwin) {
     const int lane = threadIdx.x & 31;
-    constexpr int U = 8;
     for (int64_t win = blockIdx.x; win < nwin; win += gridDim.x) {
         const int64_t s = win * 8 + (threadIdx.x >> 5);
         const int32_t row = a.srow[s * 32 + lane];
         if (row < 0) continue;
-        const int64_t b = a.soff[s];
-        const int L = (int)((a.soff[s + 1] - b) / 32);
-        const float2 yp = Y2[row];
-        const int32_t* __restrict__ c = a.scols + b + lane;
-        const float* __restrict__ w = a.sw + b + lane;
-        float lu = 0.f, lv = 0.f;
-        // the column stream runs one chunk ahead of the gathers
-        int32_t qn[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) qn[u] = u < L ? c[(int64_t)u * 32] : 0;
-        for (int j0 = 0; j0 < L; j0 += U) {
-            float2 y[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) y[u] = j0 + u < L ? Y2[qn[u]] : yp;
-            float wq[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int j = j0 + u;
-                qn[u] = j + U < L ? c[(int64_t)(j + U) * 32] : 0;
-                wq[u] = j < L ? w[(int64_t)j * 32] : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                lu = fmaf(wq[u], y[u].x - yp.x, lu);
-                lv = fmaf(wq[u], y[u].y - yp.y, lv);
-            }
-        }
-        stage_update(a, row, yp.x, yp.y, lu, lv);
+        if (a.narrow.d && a.narrow.flag[s])
+            gs_stage_slice<true>(a, s, lane, row);
+        else
+            gs_stage_slice<false>(a, s, lane, row);
     }
 }
 
@@ -282,41 +333,50 @@ __global__ void __launch_bounds__(256) gs_adjoint_kernel(RkAdjArgs<T> a) {
 // FP32 adjoint stage on the sliced ELL layout of the transposed weights: a
 // row per thread, 8 gathers of (kbar_u, kbar_v) pairs in flight; entries past
 // the slice end add the row's own pair with weight 0 (an exact zero)
-__global__ void __launch_bounds__(256) gs_adjoint_sell_kernel(RkAdjArgs<float> a, int64_t nwin) {
+template <bool C16>
+__device__ __forceinline__ void gs_adjoint_slice(const RkAdjArgs<float>& a, int64_t s, int lane, int32_t p) {
     const float2* __restrict__ KB = static_cast<const float2*>(a.pack);
+    constexpr int U = kGsEntries;
+    const int64_t b = a.soff[s];
+    const int L = (int)((a.soff[s + 1] - b) / 32);
+    SliceCols<C16, U> col(a.scols, a.narrow, b, s, lane, p);
+    const float* __restrict__ w = a.sw + b + lane;
+    float lu = 0.f, lv = 0.f;
+    // columns and weights run one chunk ahead of the gathers
+    float wn[U];
+    col.load(0, L);
+#pragma unroll
+    for (int u = 0; u < U; ++u) wn[u] = u < L ? w[(int64_t)u * 32] : 0.f;
+    for (int j0 = 0; j0 < L; j0 += U) {
+        float2 y[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) y[u] = KB[col[u]];
+        float wq[U];
+        col.load(j0 + U, L);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            wq[u] = wn[u];
+            wn[u] = j0 + U + u < L ? w[(int64_t)(j0 + U + u) * 32] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            lu = fmaf(wq[u], y[u].x, lu);
+            lv = fmaf(wq[u], y[u].y, lv);
+        }
+    }
+    adj_finish<float>(a, p, lu, lv);
+}
+
+__global__ void __launch_bounds__(256, 4) gs_adjoint_sell_kernel(RkAdjArgs<float> a, int64_t nwin) {
     const int lane = threadIdx.x & 31;
-    constexpr int U = 8;
     for (int64_t win = blockIdx.x; win < nwin; win += gridDim.x) {
         const int64_t s = win * 8 + (threadIdx.x >> 5);
         const int32_t p = a.srow[s * 32 + lane];
         if (p < 0) continue;
-        const int64_t b = a.soff[s];
-        const int L = (int)((a.soff[s + 1] - b) / 32);
-        const int32_t* __restrict__ c = a.scols + b + lane;
-        const float* __restrict__ w = a.sw + b + lane;
-        float lu = 0.f, lv = 0.f;
-        // the column stream runs one chunk ahead of the gathers
-        int32_t qn[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) qn[u] = u < L ? c[(int64_t)u * 32] : p;
-        for (int j0 = 0; j0 < L; j0 += U) {
-            float2 y[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) y[u] = KB[qn[u]];
-            float wq[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int j = j0 + u;
-                qn[u] = j + U < L ? c[(int64_t)(j + U) * 32] : p;
-                wq[u] = j < L ? w[(int64_t)j * 32] : 0.f;
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                lu = fmaf(wq[u], y[u].x, lu);
-                lv = fmaf(wq[u], y[u].y, lv);
-            }
-        }
-        adj_finish<float>(a, p, lu, lv);
+        if (a.narrow.d && a.narrow.flag[s])
+            gs_adjoint_slice<true>(a, s, lane, p);
+        else
+            gs_adjoint_slice<false>(a, s, lane, p);
     }
 }
 

@@ -143,6 +143,46 @@ __global__ void __launch_bounds__(256) sell_fill_kernel(const int64_t* __restric
     }
 }
 
+// The 16-bit columns of every slice (NarrowCols): a warp per slice, the four
+// entries of a base at a time
+__global__ void __launch_bounds__(256) sell_narrow_kernel(const int32_t* __restrict__ srow,
+                                                          const int64_t* __restrict__ off,
+                                                          const int32_t* __restrict__ cols, int64_t nslices,
+                                                          NarrowCols nc) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s < nslices; s += nwarps) {
+        const int32_t row = srow[s * kSlice + lane];
+        const int64_t b = off[s];
+        const int L = (int)((off[s + 1] - b) / kSlice);
+        int32_t* base = nc.base + narrow_base(b, s);
+        bool fits = true;
+        for (int j0 = 0; j0 < L; j0 += 4) {
+            int32_t c[4];
+            int lo = INT32_MAX, hi = INT32_MIN;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                c[u] = j0 + u < L ? cols[b + (int64_t)(j0 + u) * kSlice + lane] : row;
+                if (row < 0) c[u] = row;
+                if (c[u] != row) {
+                    lo = min(lo, c[u]);
+                    hi = max(hi, c[u]);
+                }
+            }
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            if (lo > hi) lo = hi = 0;  // every entry is its row
+            fits = fits && hi - lo <= 65534;
+            if (lane == 0) base[j0 / 4] = lo;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (j0 + u < L)
+                    nc.d[b + (int64_t)(j0 + u) * kSlice + lane] = c[u] == row ? (uint16_t)0xffffu : (uint16_t)(c[u] - lo);
+        }
+        if (lane == 0) nc.flag[s] = fits ? 1 : 0;
+    }
+}
+
 // FP64 weights on the same slices: warp per slice, 16 entries at a time
 // through a [16][33] block of doubles per warp (coalesced reads and writes)
 __global__ void __launch_bounds__(256) sell_fill64_kernel(const int64_t* __restrict__ rowptr,
@@ -255,7 +295,8 @@ constexpr bool kPipeColumns =
 // One slice: lane `lane` sums row `row` (a position, -1 past the last row)
 // over the slice's entries into acc (and, with BOUND, its weight-rounding
 // bound into bs).
-template <int NO, int U, int RK, bool BOUND, bool STREAM>
+// C16: its columns from the 16-bit stream.
+template <int NO, int U, int RK, bool BOUND, bool STREAM, bool C16>
 __device__ __forceinline__ void sell_slice(const SellArgs& a, int64_t s, int lane, int32_t row,
                                            RowAcc<NO, (RK != 0), (RK == 2)>& acc, float (&bs)[NO]) {
     const int64_t b = a.off[s];
@@ -268,6 +309,30 @@ __device__ __forceinline__ void sell_slice(const SellArgs& a, int64_t s, int lan
 #pragma unroll
     for (int o = 0; o < NO; ++o) bs[o] = 0.0f;
     const int32_t* __restrict__ c = a.cols + b + lane;
+    const uint16_t* __restrict__ c16 = C16 ? a.narrow.d + b + lane : nullptr;
+    const int32_t* __restrict__ cb = C16 ? a.narrow.base + narrow_base(b, s) : nullptr;
+    const int32_t self = max(row, 0);
+    static_assert(!C16 || U % 4 == 0, "a base serves four entries");
+    // the columns of entries [j0, min(j0 + U, L)), raw: 16-bit ones are decoded
+    // when used, so that loading ahead does not wait
+    auto load_columns = [&](int j0, int32_t (&raw)[U], int32_t (&rb)[(U + 3) / 4]) {
+        if constexpr (C16) {
+#pragma unroll
+            for (int u = 0; u < U; u += 4) rb[u / 4] = j0 + u < L ? cb[(j0 >> 2) + (u >> 2)] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int64_t at = (int64_t)(j0 + u) * kSlice;
+            if constexpr (C16)
+                raw[u] = j0 + u < L ? (int32_t)ld_stream<STREAM>(c16 + at) : 0xffff;
+            else
+                raw[u] = j0 + u < L ? ld_stream<STREAM>(c + at) : 0;
+        }
+    };
+    auto column = [&](const int32_t (&raw)[U], const int32_t (&rb)[(U + 3) / 4], int u) -> int32_t {
+        if constexpr (C16) return raw[u] == 0xffff ? self : rb[u / 4] + raw[u];
+        return raw[u];
+    };
     const float* __restrict__ w = a.w + b + lane;
     // residual streams: bf16 (RK 1) or FP32 (RK 2, the weight pairs)
     const __nv_bfloat16* __restrict__ rr = RK == 1 ? a.r + b + lane : nullptr;
@@ -276,13 +341,9 @@ __device__ __forceinline__ void sell_slice(const SellArgs& a, int64_t s, int lan
     // field gathers are issued beside its weight loads, not after a round
     // trip for its columns
     constexpr bool PIPE = kPipeColumns<NO, RK, BOUND>;
-    int32_t qn[PIPE ? U : 1];
-    if constexpr (PIPE) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) qn[u] = u < L ? ld_stream<STREAM>(c + (int64_t)u * kSlice) : 0;
-    }
+    int32_t q[U], qb[(U + 3) / 4];
+    if constexpr (PIPE) load_columns(0, q, qb);
     for (int j0 = 0; j0 < L; j0 += U) {
-        int32_t q[U];
         float wv[U][NO], rv[U][NO];
         // entries past the slice end take the row's own value (a zero
         // difference; zero for interpolation) with weight 0: no gather
@@ -293,7 +354,6 @@ __device__ __forceinline__ void sell_slice(const SellArgs& a, int64_t s, int lan
             for (int u = 0; u < U; ++u) {
                 const int j = j0 + u;
                 const bool ok = j < L;
-                if constexpr (!PIPE) q[u] = ok ? ld_stream<STREAM>(c + (int64_t)j * kSlice) : 0;
 #pragma unroll
                 for (int o = 0; o < NO; ++o) {
                     wv[u][o] = ok ? ld_stream<STREAM>(w + (int64_t)o * a.total + (int64_t)j * kSlice) : 0.0f;
@@ -311,18 +371,15 @@ __device__ __forceinline__ void sell_slice(const SellArgs& a, int64_t s, int lan
         if constexpr (PIPE) {
             // gathers of this chunk, columns of the next, then the weights
 #pragma unroll
-            for (int u = 0; u < U; ++u) fq[u] = j0 + u < L ? fld[qn[u]] : fp;
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int j = j0 + U + u;
-                qn[u] = j < L ? ld_stream<STREAM>(c + (int64_t)j * kSlice) : 0;
-            }
+            for (int u = 0; u < U; ++u) fq[u] = j0 + u < L ? fld[column(q, qb, u)] : fp;
+            load_columns(j0 + U, q, qb);
             load_weights();
         } else {
             // columns and weights, then the gathers
+            load_columns(j0, q, qb);
             load_weights();
 #pragma unroll
-            for (int u = 0; u < U; ++u) fq[u] = j0 + u < L ? fld[q[u]] : fp;
+            for (int u = 0; u < U; ++u) fq[u] = j0 + u < L ? fld[column(q, qb, u)] : fp;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) acc.add(wv[u], rv[u], fq[u], fp, a.comp);
@@ -353,8 +410,8 @@ __device__ __forceinline__ double sell_value(const RowAcc<NO, (RK != 0), (RK == 
 // B_o = sum_q |w_o,pq| |f_q - f_p| (FP32), stored to bnd[o * n + r], and the
 // largest |output| of the call per output, atomically maxed into maxabs[o]
 // (float bits; the values are >= 0, so unsigned order is float order).
-template <int NO, int U, int RK, bool BOUND, bool STREAM>
-__global__ void __launch_bounds__(256, (NO <= 3 && RK == 0 && !BOUND ? 5 : (NO <= 6 ? 4 : 3)))
+template <int NO, int U, int RK, bool BOUND, bool STREAM, bool C16>
+__global__ void __launch_bounds__(256, (NO <= (C16 ? 2 : 3) && RK == 0 && !BOUND ? 5 : (NO <= 6 ? 4 : 3)))
     apply_sell_kernel(SellArgs a) {
     // the window's outputs, staged so that they leave in row order (rows of a
     // slice are permuted; scattered 8-byte stores are slow, above all into
@@ -369,7 +426,10 @@ __global__ void __launch_bounds__(256, (NO <= 3 && RK == 0 && !BOUND ? 5 : (NO <
         const int32_t row = a.srow[s * kSlice + lane];
         RowAcc<NO, (RK != 0), (RK == 2)> acc;
         float bs[NO];
-        sell_slice<NO, U, RK, BOUND, STREAM>(a, s, lane, row, acc, bs);
+        if (C16 && a.narrow.flag[s])
+            sell_slice<NO, U, RK, BOUND, STREAM, C16>(a, s, lane, row, acc, bs);
+        else
+            sell_slice<NO, U, RK, BOUND, STREAM, false>(a, s, lane, row, acc, bs);
         if (row >= 0) {
 #pragma unroll
             for (int o = 0; o < NO; ++o) {
@@ -422,7 +482,7 @@ __global__ void __launch_bounds__(256, (NO <= 3 && RK == 0 && !BOUND ? 5 : (NO <
 // skipped when the stored maximum is already larger).
 // (launch bounds as the tile kernel's, but three blocks per SM for the bound
 // pass of six outputs, which spills at four)
-template <int NO, int U, int RK, bool BOUND, bool STREAM>
+template <int NO, int U, int RK, bool BOUND, bool STREAM, bool C16>
 __global__ void __launch_bounds__(256, (NO <= 3 && RK == 0 && !BOUND ? 5 : (NO < 6 || (NO == 6 && !BOUND) ? 4 : 3)))
     apply_sell_dyn_kernel(SellArgs a) {
     const int lane = threadIdx.x & 31;
@@ -435,7 +495,10 @@ __global__ void __launch_bounds__(256, (NO <= 3 && RK == 0 && !BOUND ? 5 : (NO <
         const int32_t row = a.srow[s * kSlice + lane];
         RowAcc<NO, (RK != 0), (RK == 2)> acc;
         float bs[NO];
-        sell_slice<NO, U, RK, BOUND, STREAM>(a, s, lane, row, acc, bs);
+        if (C16 && a.narrow.flag[s])
+            sell_slice<NO, U, RK, BOUND, STREAM, C16>(a, s, lane, row, acc, bs);
+        else
+            sell_slice<NO, U, RK, BOUND, STREAM, false>(a, s, lane, row, acc, bs);
         if (row >= 0) {
             const int64_t lr = a.perm ? (int64_t)a.perm[row] : row;
 #pragma unroll
@@ -602,6 +665,14 @@ cudaError_t sell_order(const int64_t* rowptr, int64_t n, int32_t* srow, int32_t*
     return exclusive_scan_i32(slen32, nwin * kSlicesPerWin, off, scan_tmp, s);
 }
 
+cudaError_t sell_narrow(const int32_t* srow, const int64_t* off, const int32_t* cols, int64_t nslices,
+                        const NarrowCols& nc, cudaStream_t s) {
+    if (nslices == 0) return cudaSuccess;
+    const int grid = (int)std::min<int64_t>((nslices + 7) / 8, (int64_t)num_sms() * 8);
+    sell_narrow_kernel<<<grid, 256, 0, s>>>(srow, off, cols, nslices, nc);
+    return cudaGetLastError();
+}
+
 cudaError_t sell_fill(const int64_t* rowptr, const int32_t* cols, const float* w, const void* r16, int64_t ws,
                       int nout, int64_t n, int one_set, const int32_t* srow, const int64_t* off, int64_t total,
                       int32_t* scols, float* sw, void* sr16, cudaStream_t s, const int32_t* perm,
@@ -678,31 +749,36 @@ void launch_sell(const SellArgs& a, unsigned grid, cudaStream_t s) {
     constexpr int U = NO == 1 ? 8 : 4;
     if (a.counter) {
         const int64_t slices = (a.w1 - a.w0) * kSlicesPerWin;
-#define DCPSE_DYN(UU, RK, B) \
-    apply_sell_dyn_kernel<NO, UU, RK, B, ST><<<dyn_grid<apply_sell_dyn_kernel<NO, UU, RK, B, ST>>(slices), 256, 0, s>>>(a)
+#define DCPSE_DYN(UU, RK, B, C16)                   \
+    apply_sell_dyn_kernel<NO, UU, RK, B, ST, C16>   \
+        <<<dyn_grid<apply_sell_dyn_kernel<NO, UU, RK, B, ST, C16>>(slices), 256, 0, s>>>(a)
         if (a.r32)
-            DCPSE_DYN(UR, 2, false);
+            DCPSE_DYN(UR, 2, false, false);
         else if (a.r && a.bnd)
-            DCPSE_DYN(UR, 1, true);
+            DCPSE_DYN(UR, 1, true, false);
         else if (a.r)
-            DCPSE_DYN(UR, 1, false);
+            DCPSE_DYN(UR, 1, false, false);
         else if (a.bnd)
-            DCPSE_DYN(U, 0, true);
+            DCPSE_DYN(U, 0, true, false);
+        else if (a.narrow.d)
+            DCPSE_DYN(U, 0, false, true);
         else
-            DCPSE_DYN(U, 0, false);
+            DCPSE_DYN(U, 0, false, false);
 #undef DCPSE_DYN
         return;
     }
     if (a.r32)
-        apply_sell_kernel<NO, UR, 2, false, ST><<<grid, 256, 0, s>>>(a);
+        apply_sell_kernel<NO, UR, 2, false, ST, false><<<grid, 256, 0, s>>>(a);
     else if (a.r && a.bnd)
-        apply_sell_kernel<NO, UR, 1, true, ST><<<grid, 256, 0, s>>>(a);
+        apply_sell_kernel<NO, UR, 1, true, ST, false><<<grid, 256, 0, s>>>(a);
     else if (a.r)
-        apply_sell_kernel<NO, UR, 1, false, ST><<<grid, 256, 0, s>>>(a);
+        apply_sell_kernel<NO, UR, 1, false, ST, false><<<grid, 256, 0, s>>>(a);
     else if (a.bnd)
-        apply_sell_kernel<NO, U, 0, true, ST><<<grid, 256, 0, s>>>(a);
+        apply_sell_kernel<NO, U, 0, true, ST, false><<<grid, 256, 0, s>>>(a);
+    else if (a.narrow.d)
+        apply_sell_kernel<NO, U, 0, false, ST, true><<<grid, 256, 0, s>>>(a);
     else
-        apply_sell_kernel<NO, U, 0, false, ST><<<grid, 256, 0, s>>>(a);
+        apply_sell_kernel<NO, U, 0, false, ST, false><<<grid, 256, 0, s>>>(a);
 }
 }  // namespace
 
