@@ -455,6 +455,7 @@ struct dcpse_plan_s {
     int32_t *tsell_row = nullptr, *tsell_cols = nullptr;
     int64_t* tsell_off = nullptr;
     float* tsell_w = nullptr;
+    int64_t tsell_total = 0;
     void free_tsell() {
         dfree(tsell_row);
         dfree(tsell_cols);
@@ -1972,30 +1973,39 @@ int dcpse_rk4_gs_adjoint_prepare(dcpse_plan_t* P, int precision) {
         if (!P->rs32) DCPSE_CK(dalloc(&P->rs32, P->n));
         DCPSE_CK(rk_transpose_weights<float>(P->rowptr, P->t_idx, P->n, P->nnz, P->w32, P->wT32, P->rs32, P->stream));
         // the transposed list and weights on a sliced ELL layout (the forward
-        // stage's layout, for the adjoint stage): kept only if it fits
-        P->free_tsell();
+        // stage's layout, for the adjoint stage): kept only if it fits.  The
+        // layout stays with the list, the weights are filled in every time
         if (P->n > 0) {
             const int64_t ns = sell_slices(P->n);
-            int32_t* slen = nullptr;
-            int64_t* tmp = nullptr;
-            int64_t total = 0;
-            cudaError_t e = dalloc(&P->tsell_row, (size_t)ns * 32);
-            if (e == cudaSuccess) e = dalloc(&P->tsell_off, (size_t)ns + 1);
-            if (e == cudaSuccess) e = dalloc(&slen, (size_t)ns);
-            if (e == cudaSuccess) e = dalloc(&tmp, (size_t)scan_tmp_elems(ns));
-            if (e == cudaSuccess) e = sell_order(P->t_row, P->n, P->tsell_row, slen, P->tsell_off, tmp, P->stream);
-            if (e == cudaSuccess)
-                e = cudaMemcpyAsync(&total, P->tsell_off + ns, sizeof total, cudaMemcpyDeviceToHost, P->stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(P->stream);
-            dfree(slen);
-            dfree(tmp);
-            if (e == cudaSuccess) e = dalloc(&P->tsell_cols, (size_t)total + kPad);
-            if (e == cudaSuccess) e = dalloc(&P->tsell_w, (size_t)total + kPad);
+            // (not while a stage on the plan's previous stream still reads them)
+            cudaError_t e = P->stream_changed ? cudaDeviceSynchronize() : cudaSuccess;
+            if (!P->tsell_w) {
+                P->free_tsell();
+                int32_t* slen = nullptr;
+                int64_t* tmp = nullptr;
+                int64_t total = 0;
+                e = dalloc(&P->tsell_row, (size_t)ns * 32);
+                if (e == cudaSuccess) e = dalloc(&P->tsell_off, (size_t)ns + 1);
+                if (e == cudaSuccess) e = dalloc(&slen, (size_t)ns);
+                if (e == cudaSuccess) e = dalloc(&tmp, (size_t)scan_tmp_elems(ns));
+                if (e == cudaSuccess) e = sell_order(P->t_row, P->n, P->tsell_row, slen, P->tsell_off, tmp, P->stream);
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(&total, P->tsell_off + ns, sizeof total, cudaMemcpyDeviceToHost, P->stream);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(P->stream);
+                dfree(slen);
+                dfree(tmp);
+                P->tsell_total = total;
+                if (e == cudaSuccess) e = dalloc(&P->tsell_cols, (size_t)total + kPad);
+                if (e == cudaSuccess)
+                    e = sell_fill(P->t_row, P->t_src, nullptr, nullptr, P->nnz, 1, P->n, 1, P->tsell_row, P->tsell_off,
+                                  total, P->tsell_cols, nullptr, nullptr, P->stream);
+                if (e == cudaSuccess)
+                    e = narrow_columns(P->tsell_row, P->tsell_off, P->tsell_cols, total, ns, 1, P->tsell_narrow, P->stream);
+                if (e == cudaSuccess) e = dalloc(&P->tsell_w, (size_t)total + kPad);
+            }
             if (e == cudaSuccess)
                 e = sell_fill(P->t_row, P->t_src, P->wT32, nullptr, P->nnz, 1, P->n, 1, P->tsell_row, P->tsell_off,
-                              total, P->tsell_cols, P->tsell_w, nullptr, P->stream);
-            if (e == cudaSuccess)
-                e = narrow_columns(P->tsell_row, P->tsell_off, P->tsell_cols, total, ns, 1, P->tsell_narrow, P->stream);
+                              P->tsell_total, nullptr, P->tsell_w, nullptr, P->stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(P->stream);
             if (e != cudaSuccess) {
                 P->free_tsell();

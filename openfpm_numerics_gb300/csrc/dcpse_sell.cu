@@ -30,6 +30,7 @@
 
 #include "dcpse_internal.h"
 #include "dcpse_f32_row.cuh"
+#include "dcpse_softfp.cuh"
 
 namespace dcpse {
 namespace {
@@ -231,6 +232,9 @@ template <int NO, bool STREAM>
 __global__ void __launch_bounds__(256) apply_sell64_kernel(Sell64Args a) {
     __shared__ double tile[NO][kWin];
     const int lane = threadIdx.x & 31;
+    // the difference as a three-register dfma, from three outputs on (96^3, four
+    // outputs: 669 -> 650 us; one output 287 -> 290: its registers)
+    const Fma F;
     constexpr int U = 2;  // 38 registers at four outputs: six CTAs per SM
     for (int64_t win = blockIdx.x; win < a.nwin; win += gridDim.x) {
         const int64_t s = win * kSlicesPerWin + (threadIdx.x >> 5);
@@ -259,7 +263,7 @@ __global__ void __launch_bounds__(256) apply_sell64_kernel(Sell64Args a) {
             for (int u = 0; u < U; ++u) fq[u] = j0 + u < L ? a.f[(int64_t)q[u] * a.fs] : fp;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const double d = fq[u] - fp;
+                const double d = NO > 2 ? F.add(fq[u], -fp) : fq[u] - fp;
 #pragma unroll
                 for (int o = 0; o < NO; ++o) acc[o] = fma(wv[u][o], d, acc[o]);
             }
