@@ -164,8 +164,9 @@ __global__ void row_max_kernel(const int64_t* rowptr, int64_t n, int* maxk) {
 // last used one.
 constexpr int64_t kPad = 8;
 
-// Most bytes of the neighbour search's staging rows.
-constexpr int64_t kStageBytes = int64_t(2) << 30;
+// Most bytes of the neighbour search's staging rows (3 % of the device memory;
+// beyond, or without room for them, the two-pass search serves).
+constexpr int64_t kStageBytes = int64_t(8) << 30;
 
 // Largest scratch of one assembly batch; larger clouds are assembled in
 // batches of particles (the result does not depend on the batch size).
@@ -1463,16 +1464,26 @@ int ensure_sell64(dcpse_plan_t* P);
 
 // The plan's scratch for batches of particles of `per` bytes each, at most
 // kAsmScratchBytes (the Gram entries, coefficients and scaled offsets of the
-// particles in flight).
+// particles in flight); smaller batches where device memory is short (the
+// result does not depend on the batch size).
 int asm_batches(dcpse_plan_t* P, AsmArgs& a, int64_t per) {
-    const int64_t nb = std::min<int64_t>(a.n, std::max<int64_t>(4096, kAsmScratchBytes / per));
-    const int64_t bytes = nb * per + 16;
-    if (P->asm_scratch_bytes < bytes) {
+    int64_t nb = std::min<int64_t>(a.n, std::max<int64_t>(4096, kAsmScratchBytes / per));
+    cudaError_t e = cudaSuccess;
+    while (P->asm_scratch_bytes < nb * per + 16) {
+        const int64_t bytes = nb * per + 16;
         dfree(P->asm_scratch);
         P->asm_scratch_bytes = 0;
-        DCPSE_CK(dalloc(&P->asm_scratch, (size_t)(bytes + 7) / 8));
-        P->asm_scratch_bytes = bytes;
+        e = dalloc(&P->asm_scratch, (size_t)(bytes + 7) / 8);
+        if (e == cudaSuccess) {
+            P->asm_scratch_bytes = bytes;
+        } else if (e == cudaErrorMemoryAllocation && nb > 4096) {
+            cudaGetLastError();
+            nb = std::max<int64_t>(4096, nb / 2);
+        } else {
+            break;
+        }
     }
+    DCPSE_CK(e);
     a.scratch = P->asm_scratch;
     a.scratch_particles = nb;
     return DCPSE_OK;
