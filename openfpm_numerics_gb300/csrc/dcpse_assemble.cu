@@ -5,10 +5,11 @@
 // 620-717: per-thread global scratch B, cuBLAS batched LU without pivoting,
 // a separate calcKernels_gpu pass and host round trips).
 //
-// Particles are assembled in batches, each by three kernels that hand their
-// results over through a plan-owned scratch buffer:
-//  1. gram_kernel (one warp per particle)
+// eps_kernel (a thread per particle) forms
 //       eps  = (sum_q sum_d |x_pq,d|) / k / HOverEpsilon   (Vandermonde.hpp:63-81)
+// for every particle.  Particles are then assembled in batches, each by three
+// kernels that hand their results over through a plan-owned scratch buffer:
+//  1. gram_kernel (one warp per particle)
 //       Gram A_ij = sum_q B_qi B_qj,  B_qj = E_q V_qj,
 //            V_qj = m_j(x_pq/eps), E_q = exp(-|x_pq|^2 / (2 eps^2))
 //            (Vandermonde.hpp:36-49, DcpseDiagonalScalingMatrix.hpp:21-41,
@@ -25,8 +26,11 @@
 //       square root, divisions); with few lanes per particle one warp
 //       instruction advances many particles, which is what the FP64 pipe of
 //       this part needs.  Coefficients go back to scratch.
-//  3. weights_kernel (one warp per particle)
+//  3. weights_kernel (a warp takes a run of particles, its lanes their
+//       concatenated neighbour rows)
 //       K_q = exp(-|x_pq/eps|^2) sum_i a_i V_qi        (Dcpse.hpp:768-809)
+// The FP64 pipe bounds all three; products and quotients that the integer
+// pipes can round (dcpse_softfp.cuh) run there beside it, with the same bits.
 //
 // Every floating-point operation follows the order of the CPU oracle, and
 // this translation unit is compiled with -fmad=false (fused multiply-adds are

@@ -6,7 +6,10 @@
 //  * GPU: gatherSupportSize_gpu / assembleSupport_gpu with a host prefix sum
 //    (src/DCPSE/SupportBuilder.cuh:14-107).
 // Here every step stays on the device: cell ids, counting sort into cells,
-// a count pass, a device exclusive scan, a fill pass and a per-row sort.
+// one search that writes each row's neighbours to staging rows and counts them
+// (dcpse_nbr_group.cuh: candidates loaded once per group of cells), a device
+// exclusive scan and a per-row sort out of the staging rows.  Where the staging
+// rows do not fit, a count pass and a fill pass over the candidates serve.
 // The list of particle p is every q != p with |x_p - x_q|^2 < rc_p^2 in
 // ascending q, so it does not depend on the cell size or on the order in
 // which atomics filled the cells.
