@@ -12,13 +12,12 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
-#include <mutex>
 #include <string>
-#include <unordered_map>
 #include <utility>
 #include <vector>
 
 #include "dcpse_internal.h"
+#include "dcpse_memory.h"
 
 using namespace dcpse;
 
@@ -172,141 +171,15 @@ constexpr int64_t kStageBytes = int64_t(8) << 30;
 // batches of particles (the result does not depend on the batch size).
 constexpr int64_t kAsmScratchBytes = int64_t(512) << 20;
 
-// Device memory of the plans.  A freed block is kept for the next request of
-// about its size instead of going back to the driver, whose cudaMalloc and
-// cudaFree cost 10 us to 1 ms each (a neighbour build makes 14 of each, an
-// operator update of 4,096 particles spent 0.6 of its 1.0 ms there).  Shared by
-// all plans and threads of the process, since an operator update builds its list
-// on a plan of its own.  Bounded: at most kPoolBytes of free blocks per process,
-// given back when a request cannot be met and when the last plan is destroyed.
-// cudaFree waits for the device; here a block is handed out again only after a
-// device synchronisation later than its release, so whatever stream or thread
-// still used it when it was freed has finished.
-thread_local cudaStream_t t_plan_stream = nullptr;  // stream of the plan this thread works on (check_plan)
-
-class DevicePool {
-public:
-    cudaError_t alloc(void** p, size_t want) {
-        *p = nullptr;
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e != cudaSuccess) return e;
-        size_t bytes = rounded(want);
-        unsigned long long wait = 0;
-        {
-            std::lock_guard<std::mutex> lock(m_);
-            if (take(p, dev, bytes, synced_[dev])) return cudaSuccess;
-            if (find(dev, bytes, ~0ull) != free_.end()) wait = stamp_;
-        }
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        if (wait && (cudaStreamIsCapturing(t_plan_stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) {
-            cudaGetLastError();
-            wait = 0;  // inside a stream capture: as without a pool
-        }
-        if (wait) {
-            // released, but perhaps still in use: after a synchronisation not
-            if (cudaDeviceSynchronize() == cudaSuccess) {
-                std::lock_guard<std::mutex> lock(m_);
-                synced_[dev] = std::max(synced_[dev], wait);
-                if (take(p, dev, bytes, synced_[dev])) return cudaSuccess;
-            }
-        }
-        e = cudaMalloc(p, bytes);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            release();
-            bytes = want;
-            e = cudaMalloc(p, bytes);
-        }
-        if (e == cudaSuccess) {
-            std::lock_guard<std::mutex> lock(m_);
-            live_[*p] = Block{bytes, dev, 0};
-        } else {
-            *p = nullptr;
-        }
-        return e;
-    }
-    void free(void* p) {
-        if (!p) return;
-        {
-            std::lock_guard<std::mutex> lock(m_);
-            auto it = live_.find(p);
-            if (it != live_.end()) {
-                Block b = it->second;
-                live_.erase(it);
-                if (cached_ + b.bytes <= kPoolBytes) {
-                    b.stamp = ++stamp_;
-                    cached_ += b.bytes;
-                    free_.emplace(b.bytes, std::make_pair(p, b));
-                    return;
-                }
-            }
-        }
-        cudaFree(p);
-    }
-    void plan_created() {
-        std::lock_guard<std::mutex> lock(m_);
-        ++plans_;
-    }
-    void plan_destroyed() {
-        bool last;
-        {
-            std::lock_guard<std::mutex> lock(m_);
-            last = --plans_ == 0;
-        }
-        if (last) release();
-    }
-    // every free block back to the driver
-    void release() {
-        std::vector<std::pair<void*, int>> blocks;
-        {
-            std::lock_guard<std::mutex> lock(m_);
-            for (auto& f : free_) blocks.emplace_back(f.second.first, f.second.second.dev);
-            free_.clear();
-            cached_ = 0;
-        }
-        for (auto& b : blocks) cudaFree(b.first);  // (any device's: pointers are unified)
-    }
-
-private:
-    static constexpr size_t kPoolBytes = size_t(4) << 30;
-    struct Block {
-        size_t bytes;
-        int dev;
-        unsigned long long stamp;  // order of the releases
-    };
-    // sixteenths of a power of two, at least 512 bytes: lists and weights of
-    // moving particles change a little in size from step to step
-    static size_t rounded(size_t want) {
-        size_t unit = 512;
-        while (unit * 32 <= want) unit *= 2;
-        return (want + unit - 1) / unit * unit;
-    }
-    using FreeMap = std::multimap<size_t, std::pair<void*, Block>>;
-    // a free block of this device of `bytes` or up to an eighth more, released
-    // before the device's last known synchronisation
-    FreeMap::iterator find(int dev, size_t bytes, unsigned long long synced) {
-        for (auto it = free_.lower_bound(bytes); it != free_.end() && it->first <= bytes + bytes / 8; ++it)
-            if (it->second.second.dev == dev && it->second.second.stamp <= synced) return it;
-        return free_.end();
-    }
-    bool take(void** p, int dev, size_t bytes, unsigned long long synced) {
-        auto it = find(dev, bytes, synced);
-        if (it == free_.end()) return false;
-        *p = it->second.first;
-        live_[*p] = it->second.second;
-        cached_ -= it->first;
-        free_.erase(it);
-        return true;
-    }
-    std::mutex m_;
-    std::unordered_map<void*, Block> live_;
-    FreeMap free_;
-    std::unordered_map<int, unsigned long long> synced_;
-    unsigned long long stamp_ = 0;
-    size_t cached_ = 0;
-    int plans_ = 0;
+struct CudaRt {
+    typedef cudaError_t Error;
+    static constexpr cudaError_t ok = cudaSuccess, no_memory = cudaErrorMemoryAllocation;
+    static Error malloc(void** p, size_t bytes) { return cudaMalloc(p, bytes); }
+    static Error free(void* p) { return cudaFree(p); }
+    static Error device(int* dev) { return cudaGetDevice(dev); }
+    static void clear_error() { cudaGetLastError(); }
 };
+typedef DevicePoolT<CudaRt> DevicePool;
 
 // (never destroyed: plans may outlive static destructors)
 DevicePool& pool() {
@@ -845,7 +718,6 @@ Geom plan_geom(const dcpse_plan_s* P) {
 
 int check_plan(dcpse_plan_t* P) {
     if (!P) return fail(DCPSE_ERR_ARG, "null plan");
-    t_plan_stream = P->stream;
     return DCPSE_OK;
 }
 
@@ -1024,7 +896,6 @@ int dcpse_plan_create(dcpse_plan_t** plan, int dim, int n_outputs, const int* te
                       const unsigned* signatures, unsigned order, double h_over_eps) {
     if (!plan) return fail(DCPSE_ERR_ARG, "plan is NULL");
     *plan = nullptr;
-    t_plan_stream = nullptr;
     if (dim < 1 || dim > 3) return fail(DCPSE_ERR_ARG, "dim must be 1, 2 or 3");
     if (n_outputs < 1 || n_outputs > kMaxOutputs) return fail(DCPSE_ERR_CAPACITY, "1..8 outputs per plan");
     if (!terms_per_output || !signatures) return fail(DCPSE_ERR_ARG, "NULL terms/signatures");
@@ -1521,7 +1392,7 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
     if (!(flags & DCPSE_STORE_OUT_F64)) dfree(P->w64);
     // the weights are rewritten (a surface operator's list, too): not while
     // an apply on the plan's previous stream still reads them
-    if (P->stream_changed) DCPSE_CK(cudaDeviceSynchronize());
+    if (P->stream_changed) DCPSE_CK(pool().wait());
     P->stream_changed = false;
     if (P->surface())
         P->free_sell();
@@ -1989,7 +1860,7 @@ int dcpse_rk4_gs_adjoint_prepare(dcpse_plan_t* P, int precision) {
         if (P->n > 0) {
             const int64_t ns = sell_slices(P->n);
             // (not while a stage on the plan's previous stream still reads them)
-            cudaError_t e = P->stream_changed ? cudaDeviceSynchronize() : cudaSuccess;
+            cudaError_t e = P->stream_changed ? pool().wait() : cudaSuccess;
             if (!P->tsell_w) {
                 P->free_tsell();
                 int32_t* slen = nullptr;
