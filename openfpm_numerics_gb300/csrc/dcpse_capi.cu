@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <array>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -190,6 +191,10 @@ DevicePool& pool() {
 template <typename T>
 cudaError_t dalloc(T** p, size_t count) {
     if (count == 0) count = 1;
+    if (count > SIZE_MAX / sizeof(T)) {  // (a caller's absurd size must not wrap around to a small one)
+        *p = nullptr;
+        return cudaErrorMemoryAllocation;
+    }
     return pool().alloc((void**)p, count * sizeof(T));
 }
 cudaError_t dalloc_bytes(void** p, size_t bytes) { return pool().alloc(p, bytes ? bytes : 1); }
@@ -2080,10 +2085,10 @@ int dcpse_apply_output_f64(dcpse_plan_t* P, int output, const double* d_f, doubl
     if (!P->assembled || !P->k_term) return fail(DCPSE_ERR_STATE, "per-term FP64 kernels not stored");
     if (output < 0 || output >= P->nout) return fail(DCPSE_ERR_ARG, "output out of range");
     if (P->n > 0 && (!d_f || !d_out)) return fail(DCPSE_ERR_ARG, "NULL field");
-    std::vector<int> terms;
+    int terms[kMaxTerms], count = 0;
     for (int t = 0; t < P->nterms; ++t)
-        if (P->term_output[t] == output) terms.push_back(t);
-    return apply_terms(P, terms.data(), (int)terms.size(), d_f, d_out);
+        if (P->term_output[t] == output) terms[count++] = t;
+    return apply_terms(P, terms, count, d_f, d_out);
 }
 
 namespace {

@@ -25,7 +25,6 @@
 #include <mutex>
 #include <unordered_map>
 #include <utility>
-#include <vector>
 
 namespace dcpse {
 
@@ -44,12 +43,12 @@ public:
         bool waiting = false;  // a block would do once it is known to be idle
         {
             std::lock_guard<std::mutex> lock(m_);
-            if (take(p, dev, bytes, synced_[dev])) return Rt::ok;
+            if (take(p, dev, bytes)) return Rt::ok;
             waiting = find(dev, bytes, ~0ull) != free_.end();
         }
         if (waiting && wait() == Rt::ok) {
             std::lock_guard<std::mutex> lock(m_);
-            if (take(p, dev, bytes, synced_[dev])) return Rt::ok;
+            if (take(p, dev, bytes)) return Rt::ok;
         }
         e = Rt::malloc(p, bytes);
         if (e == Rt::no_memory) {
@@ -59,8 +58,8 @@ public:
             e = Rt::malloc(p, bytes);
         }
         if (e == Rt::ok) {
-            std::lock_guard<std::mutex> lock(m_);
-            live_[*p] = Block{bytes, dev, 0};
+            // (a block that cannot be noted goes back to the driver when freed)
+            noted([&] { live_[*p] = Block{bytes, dev, 0}; });
         } else {
             *p = nullptr;
         }
@@ -68,21 +67,19 @@ public:
     }
     void free(void* p) {
         if (!p) return;
-        {
-            std::lock_guard<std::mutex> lock(m_);
+        bool kept = false;
+        noted([&] {
             auto it = live_.find(p);
-            if (it != live_.end()) {
-                Block b = it->second;
-                live_.erase(it);
-                if (cached_ + b.bytes <= kPoolBytes) {
-                    b.stamp = ++stamp_;
-                    cached_ += b.bytes;
-                    free_.emplace(b.bytes, std::make_pair(p, b));
-                    return;
-                }
-            }
-        }
-        Rt::free(p);
+            if (it == live_.end()) return;
+            Block b = it->second;
+            live_.erase(it);
+            if (cached_ + b.bytes > kPoolBytes) return;
+            b.stamp = ++stamp_;
+            free_.emplace(b.bytes, std::make_pair(p, b));
+            cached_ += b.bytes;
+            kept = true;
+        });
+        if (!kept) Rt::free(p);
     }
     // What cudaFree does beside freeing: returns when the work that was submitted
     // to the current device, on any stream, is done.
@@ -98,12 +95,10 @@ public:
         void* p = nullptr;
         e = Rt::malloc(&p, 1);
         if (e == Rt::ok) e = Rt::free(p);
-        if (e == Rt::ok) {
-            std::lock_guard<std::mutex> lock(m_);
-            synced_[dev] = std::max(synced_[dev], stamp);
-        } else {
+        if (e == Rt::ok)
+            noted([&] { synced_[dev] = std::max(synced_[dev], stamp); });
+        else
             Rt::clear_error();
-        }
         return e;
     }
     void plan_created() {
@@ -120,14 +115,13 @@ public:
     }
     // every free block back to the driver
     void release() {
-        std::vector<void*> blocks;
+        FreeMap blocks;
         {
             std::lock_guard<std::mutex> lock(m_);
-            for (auto& f : free_) blocks.push_back(f.second.first);
-            free_.clear();
+            blocks.swap(free_);
             cached_ = 0;
         }
-        for (void* p : blocks) Rt::free(p);  // (any device's: pointers are unified)
+        for (auto& f : blocks) Rt::free(f.second.first);  // (any device's: pointers are unified)
     }
 
 private:
@@ -136,14 +130,26 @@ private:
         int dev;
         unsigned long long stamp;  // order of the releases
     };
+    using FreeMap = std::multimap<size_t, std::pair<void*, Block>>;
+    // fn under the lock; its bookkeeping may fail for want of host memory, which
+    // must not leave a C entry point as an exception
+    template <class Fn>
+    void noted(Fn fn) {
+        std::lock_guard<std::mutex> lock(m_);
+        try {
+            fn();
+        } catch (...) {
+        }
+    }
     // sixteenths of a power of two, at least 512 bytes: lists and weights of
-    // moving particles change a little in size from step to step
+    // moving particles change a little in size from step to step (sizes that no
+    // device has are left as they are, for the driver to refuse)
     static size_t rounded(size_t want) {
+        if (want >= size_t(1) << 48) return want;
         size_t unit = 512;
         while (unit * 32 <= want) unit *= 2;
         return (want + unit - 1) / unit * unit;
     }
-    using FreeMap = std::multimap<size_t, std::pair<void*, Block>>;
     // a free block of this device of `bytes` or up to an eighth more, released
     // before the device's last known wait
     typename FreeMap::iterator find(int dev, size_t bytes, unsigned long long synced) {
@@ -151,11 +157,16 @@ private:
             if (it->second.second.dev == dev && it->second.second.stamp <= synced) return it;
         return free_.end();
     }
-    bool take(void** p, int dev, size_t bytes, unsigned long long synced) {
-        auto it = find(dev, bytes, synced);
+    bool take(void** p, int dev, size_t bytes) {
+        auto known = synced_.find(dev);
+        auto it = find(dev, bytes, known == synced_.end() ? 0ull : known->second);
         if (it == free_.end()) return false;
+        try {
+            live_[it->second.first] = it->second.second;
+        } catch (...) {
+            return false;
+        }
         *p = it->second.first;
-        live_[*p] = it->second.second;
         cached_ -= it->first;
         free_.erase(it);
         return true;

@@ -32,7 +32,7 @@ struct Fake {
         std::lock_guard<std::mutex> lock(m);
         *p = nullptr;
         if (refuse) return last_error = 900;
-        if (used + bytes > limit) return last_error = no_memory;
+        if (bytes > limit - used) return last_error = no_memory;
         used += bytes;
         *p = reinterpret_cast<void*>(next);
         next += bytes + 256;
@@ -99,7 +99,16 @@ int main() {
         CHECK(pool.wait() != 0 && Fake::last_error == 0);
         CHECK(pool.alloc(&a, 140000) != 0 && a == nullptr);
         Fake::refuse = false;
+        // sizes that no device has are refused (and end: doubling a unit up to
+        // them would wrap around)
+        Fake::limit = size_t(1) << 40;
+        for (size_t absurd : {size_t(1) << 62, size_t(1) << 63, ~size_t(0) - 7, ~size_t(0)})
+            CHECK(pool.alloc(&a, absurd) == Fake::no_memory && a == nullptr);
+        Fake::clear_error();
+        Fake::limit = ~size_t(0) / 2;
         // the last plan's end gives everything back
+        CHECK(pool.alloc(&a, 3000) == 0);
+        pool.free(a);
         pool.plan_created();
         pool.plan_created();
         pool.plan_destroyed();
