@@ -1223,8 +1223,8 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
     if (!other_support && stage_neighbors_serves(a)) {
         double ball = dim == 2 ? 3.14159265 * rmax * rmax : 4.18879020 * rmax * rmax * rmax;
         for (int d = 0; d < dim; ++d) ball /= std::max(hi[d] - lo[d], rmax);
-        const double want = std::min(1.3 * ball * (double)n + 16.0, 1024.0);
-        row_cap = ((int)want + 31) / 32 * 32;
+        const double want = 1.3 * ball * (double)n + 16.0;
+        row_cap = want < 1024.0 ? ((int)want + 31) / 32 * 32 : 1024;  // (NaN, of an infinite cutoff: 1024)
         if ((int64_t)row_cap * n * (int64_t)sizeof(int32_t) > kStageBytes || dalloc(&tmp, (size_t)row_cap * n) != cudaSuccess) {
             cudaGetLastError();
             row_cap = 0;
