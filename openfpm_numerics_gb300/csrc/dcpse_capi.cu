@@ -199,10 +199,34 @@ cudaError_t dalloc(T** p, size_t count) {
 }
 cudaError_t dalloc_bytes(void** p, size_t bytes) { return pool().alloc(p, bytes ? bytes : 1); }
 
+// Buffers given up by this thread.  Without the pool each was a cudaFree, which
+// waited for the device: the entry points that give up a plan's buffers wait once
+// instead (settle), before they write any array in place or return.  So no reader
+// of the plan's arrays on another stream is overtaken, inputs that another stream
+// still writes are complete, and a closed plan's callers may reuse theirs.
+thread_local unsigned long t_given_up = 0;
+
 template <typename T>
 void dfree(T*& p) {
-    if (p) pool().free((void*)p);
+    if (p) {
+        pool().free((void*)p);
+        ++t_given_up;
+    }
     p = nullptr;
+}
+
+int settle() {
+    DCPSE_CK(pool().wait());
+    return DCPSE_OK;
+}
+
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &c) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return c != cudaStreamCaptureStatusNone;
 }
 
 }  // namespace
@@ -437,6 +461,7 @@ struct dcpse_plan_s {
     void* spare_r = nullptr;
     void drop_sell_weights(bool f32, bool f64) {
         auto keep = [](auto& live, auto& spare, bool wanted) {
+            if (live) ++t_given_up;  // (a spare is written again, too)
             if (live && wanted && !spare)
                 spare = live;
             else if (live)
@@ -954,6 +979,7 @@ int dcpse_plan_destroy(dcpse_plan_t* P) {
     if (!P) return DCPSE_OK;
     if (P->stream) cudaStreamSynchronize(P->stream);
     P->free_all();
+    pool().wait();
     delete P;
     return DCPSE_OK;
 }
@@ -986,6 +1012,7 @@ int dcpse_plan_set_support(dcpse_plan_t* P, const double* d_pos_support, int64_t
     if (d_pos_support && n_support < 0) return fail(DCPSE_ERR_ARG, "bad support set size");
     if (d_pos_support && n_support >= (int64_t)INT32_MAX) return fail(DCPSE_ERR_CAPACITY, "at most 2^31-1 particles");
     // the neighbour list and everything assembled on it refer to the old sets
+    const unsigned long given_up = t_given_up;
     P->free_assembly();
     P->free_transpose();
     dfree(P->rowptr);
@@ -997,7 +1024,7 @@ int dcpse_plan_set_support(dcpse_plan_t* P, const double* d_pos_support, int64_t
     P->sup_pos = d_pos_support;
     P->n_sup = d_pos_support ? n_support : 0;
     P->self_skip = self_skip ? 1 : 0;
-    return DCPSE_OK;
+    return t_given_up != given_up ? settle() : DCPSE_OK;
 }
 
 int dcpse_plan_set_surface(dcpse_plan_t* P, const double* d_normals, int n_count, double n_spacing,
@@ -1005,6 +1032,7 @@ int dcpse_plan_set_surface(dcpse_plan_t* P, const double* d_normals, int n_count
     if (int rc = check_plan(P)) return rc;
     if (d_normals && n_count < 1) return fail(DCPSE_ERR_ARG, "n_count must be >= 1");
     if (d_normals && !d_n_spacings && !(n_spacing > 0.0)) return fail(DCPSE_ERR_ARG, "n_spacing must be > 0");
+    const unsigned long given_up = t_given_up;
     P->free_assembly();
     P->free_transpose();
     dfree(P->rowptr);
@@ -1019,7 +1047,7 @@ int dcpse_plan_set_surface(dcpse_plan_t* P, const double* d_normals, int n_count
     P->surf_spacing = n_spacing;
     P->surf_spacings = d_normals ? d_n_spacings : nullptr;
     P->surf_pending = false;
-    return DCPSE_OK;
+    return t_given_up != given_up ? settle() : DCPSE_OK;
 }
 
 int dcpse_plan_info(dcpse_plan_t* P, int64_t* n, int64_t* nnz, int* n_terms, int* n_outputs, int* max_neighbors) {
@@ -1057,6 +1085,7 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
     dfree(P->cell_order);
     P->list_version++;
     dfree(P->cols);
+    if (int rc = settle()) return rc;
     P->n = n;
     P->nnz = 0;
     P->maxk = 0;
@@ -1290,6 +1319,7 @@ int dcpse_set_neighbors(dcpse_plan_t* P, int64_t n, int64_t nnz, const int64_t* 
     dfree(P->cell_order);
     P->list_version++;
     dfree(P->cols);
+    if (int rc = settle()) return rc;
     P->n = n;
     P->nnz = nnz;
     DCPSE_CK(dalloc(&P->rowptr, (size_t)n + 1));
@@ -1388,6 +1418,7 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
     const int64_t n = P->n, nnz = P->nnz;
     const int ng = P->htab->ngroups;
     // (re)allocate what this assembly stores
+    const unsigned long given_up = t_given_up;
     if (!P->eps) DCPSE_CK(dalloc(&P->eps, n));
     if (!P->status) DCPSE_CK(dalloc(&P->status, n));
     if (!P->eip_group) DCPSE_CK(dalloc(&P->eip_group, (size_t)ng * n));
@@ -1395,10 +1426,7 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
     if (!(flags & DCPSE_STORE_TERMS_F64)) dfree(P->k_term);
     if ((flags & DCPSE_STORE_OUT_F64) && !P->w64) DCPSE_CK(dalloc(&P->w64, (size_t)P->nout * nnz));
     if (!(flags & DCPSE_STORE_OUT_F64)) dfree(P->w64);
-    // the weights are rewritten (a surface operator's list, too): not while
-    // an apply on the plan's previous stream still reads them
-    if (P->stream_changed) DCPSE_CK(pool().wait());
-    P->stream_changed = false;
+    // the weights are rewritten (a surface operator's list, too)
     if (P->surface())
         P->free_sell();
     else
@@ -1414,6 +1442,10 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
     if (!(flags & DCPSE_STORE_OUT_F32_RESID)) dfree(P->r16);
     if ((flags & DCPSE_STORE_OUT_F32_CORR) && !P->r32) DCPSE_CK(dalloc(&P->r32, (size_t)P->nout * nnz + kPad));
     if (!(flags & DCPSE_STORE_OUT_F32_CORR)) dfree(P->r32);
+    // not while an apply on the plan's previous stream still reads them, either
+    if (t_given_up != given_up || (P->stream_changed && !capturing(s)))
+        if (int rc = settle()) return rc;
+    P->stream_changed = false;
     AsmArgs a{};
     a.tab = P->dtab;
     a.dim = P->dim;
@@ -1554,6 +1586,7 @@ int dcpse_set_term_kernels(dcpse_plan_t* P, int term, const double* d_kernels, c
     if ((P->nnz > 0 && !d_kernels) || (P->n > 0 && (!d_eps || !d_eps_inv_pow)))
         return fail(DCPSE_ERR_ARG, "NULL array");
     const int64_t n = P->n, nnz = P->nnz;
+    const unsigned long given_up = t_given_up;
     if (!P->assembled) {
         // fresh plan (support_options::LOAD): kernels of every term start at zero
         P->free_assembly();
@@ -1579,6 +1612,8 @@ int dcpse_set_term_kernels(dcpse_plan_t* P, int term, const double* d_kernels, c
     dfree(P->rowsum);
     P->rowsum_prec = -1;
     P->free_vsell_weights();
+    if (t_given_up != given_up)
+        if (int rc = settle()) return rc;
     cudaStream_t s = P->stream;
     if (nnz > 0)
         DCPSE_CK(cudaMemcpyAsync(P->k_term + (size_t)term * nnz, d_kernels, sizeof(double) * nnz,
@@ -1856,6 +1891,9 @@ int dcpse_rk4_gs_adjoint_prepare(dcpse_plan_t* P, int precision) {
     if (int rc = ensure_transpose(P)) return rc;
     if (precision == DCPSE_F32) {
         if (!P->w32) return fail(DCPSE_ERR_STATE, "FP32 weights not stored");
+        // (not while a stage on another stream still reads them)
+        if (P->wT32 || P->rs32)
+            if (int rc = settle()) return rc;
         if (!P->wT32) DCPSE_CK(dalloc(&P->wT32, P->nnz));
         if (!P->rs32) DCPSE_CK(dalloc(&P->rs32, P->n));
         DCPSE_CK(rk_transpose_weights<float>(P->rowptr, P->t_idx, P->n, P->nnz, P->w32, P->wT32, P->rs32, P->stream));
@@ -1864,8 +1902,7 @@ int dcpse_rk4_gs_adjoint_prepare(dcpse_plan_t* P, int precision) {
         // layout stays with the list, the weights are filled in every time
         if (P->n > 0) {
             const int64_t ns = sell_slices(P->n);
-            // (not while a stage on the plan's previous stream still reads them)
-            cudaError_t e = P->stream_changed ? pool().wait() : cudaSuccess;
+            cudaError_t e = cudaSuccess;
             if (!P->tsell_w) {
                 P->free_tsell();
                 int32_t* slen = nullptr;
@@ -2621,7 +2658,10 @@ int dcpse_plan_set_reorder(dcpse_plan_t* P, int policy) {
         P->reorder = policy;
         // the sliced layouts are rebuilt on next use
         const bool had = P->sell_w != nullptr;
+        const unsigned long given_up = t_given_up;
         P->free_sell();
+        if (t_given_up != given_up)
+            if (int rc = settle()) return rc;
         if (had && P->assembled)
             if (int rc = ensure_sell(P)) return rc;
     }
