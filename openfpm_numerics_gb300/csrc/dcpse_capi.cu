@@ -351,6 +351,11 @@ struct dcpse_plan_s {
     int rowsum_prec = -1;
     double* gentry = nullptr;
     double* vjp_eps = nullptr;  // eps and eps^-|alpha| of the position VJP [1 + groups][n]
+    // its batch scratch: not the assembly's, since it needs nothing of an
+    // assembly that may still run (DCPSE_ASSEMBLE_ASYNC, another stream), and kept
+    // with the list, so that captured calls keep their addresses
+    double* vjp_scratch = nullptr;
+    int64_t vjp_scratch_bytes = 0, vjp_batch = 0;
     // transposed Laplacian weights of output 0 for the RK4 adjoint, and the
     // FP32 ones on a sliced ELL layout of the transposed list
     float *wT32 = nullptr, *rs32 = nullptr;
@@ -396,6 +401,8 @@ struct dcpse_plan_s {
         dfree(rowsum);
         dfree(gentry);
         dfree(vjp_eps);
+        dfree(vjp_scratch);
+        vjp_scratch_bytes = 0;
         dfree(wT32);
         dfree(rs32);
         dfree(wT64);
@@ -1368,20 +1375,20 @@ namespace {
 int ensure_sell(dcpse_plan_t* P);
 int ensure_sell64(dcpse_plan_t* P);
 
-// The plan's scratch for batches of particles of `per` bytes each, at most
+// Scratch for batches of particles of `per` bytes each, at most
 // kAsmScratchBytes (the Gram entries, coefficients and scaled offsets of the
 // particles in flight); smaller batches where device memory is short (the
 // result does not depend on the batch size).
-int asm_batches(dcpse_plan_t* P, AsmArgs& a, int64_t per) {
+int batch_scratch(double*& scratch, int64_t& have, AsmArgs& a, int64_t per) {
     int64_t nb = std::min<int64_t>(a.n, std::max<int64_t>(4096, kAsmScratchBytes / per));
     cudaError_t e = cudaSuccess;
-    while (P->asm_scratch_bytes < nb * per + 16) {
+    while (have < nb * per + 16) {
         const int64_t bytes = nb * per + 16;
-        dfree(P->asm_scratch);
-        P->asm_scratch_bytes = 0;
-        e = dalloc(&P->asm_scratch, (size_t)(bytes + 7) / 8);
+        dfree(scratch);
+        have = 0;
+        e = dalloc(&scratch, (size_t)(bytes + 7) / 8);
         if (e == cudaSuccess) {
-            P->asm_scratch_bytes = bytes;
+            have = bytes;
         } else if (e == cudaErrorMemoryAllocation && nb > 4096) {
             cudaGetLastError();
             nb = std::max<int64_t>(4096, nb / 2);
@@ -1390,7 +1397,7 @@ int asm_batches(dcpse_plan_t* P, AsmArgs& a, int64_t per) {
         }
     }
     DCPSE_CK(e);
-    a.scratch = P->asm_scratch;
+    a.scratch = scratch;
     a.scratch_particles = nb;
     return DCPSE_OK;
 }
@@ -1473,7 +1480,8 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
     a.err = P->d_err;
     a.order = nullptr;
     if (n > 0) {
-        if (int rc = asm_batches(P, a, assembly_scratch_bytes(*P->htab, flags, P->maxk))) return rc;
+        if (int rc = batch_scratch(P->asm_scratch, P->asm_scratch_bytes, a, assembly_scratch_bytes(*P->htab, flags, P->maxk)))
+            return rc;
         const int64_t qb = assembly_qr_ws_bytes(*P->htab, flags);
         if (qb > 0 && P->qr_ws_bytes < qb) {
             dfree(P->qr_ws);
@@ -1808,7 +1816,14 @@ int dcpse_vjp_positions(dcpse_plan_t* P, const double* d_pos, const double* d_ep
     a.gbar = d_g;
     a.gentry = P->gentry;
     a.gown = d_grad;
-    if (int rc = asm_batches(P, a, vjp_scratch_bytes(*P->htab, P->maxk))) return rc;
+    if (P->vjp_scratch) {
+        a.scratch = P->vjp_scratch;
+        a.scratch_particles = P->vjp_batch;
+    } else {
+        if (int rc = batch_scratch(P->vjp_scratch, P->vjp_scratch_bytes, a, vjp_scratch_bytes(*P->htab, P->maxk)))
+            return rc;
+        P->vjp_batch = a.scratch_particles;
+    }
     cudaError_t e = vjp_entries(a, *P->htab, P->stream);
     if (e == cudaErrorInvalidConfiguration)
         return fail(DCPSE_ERR_CAPACITY, "position VJP: the QR work space of this lane grouping exceeds shared memory");

@@ -201,3 +201,35 @@ def test_adjoint_prepared_again_on_another_stream(cuda):
     torch.cuda.synchronize()
     assert torch.equal(ref[0], got[0]) and torch.equal(ref[1], got[1])
     plan.close()
+
+
+def test_position_vjp_beside_a_pending_assembly(cuda):
+    """The position VJP needs nothing of an assembly: on another stream it may
+    run before, during or after one that is pending, and changes none of it."""
+    pos, h = W.lattice(20, 3, jitter=0.1, seed=85)
+    p = torch.tensor(pos, device="cuda")
+    rng = np.random.default_rng(85)
+    f = torch.tensor(rng.standard_normal(pos.shape[0]), device="cuda")
+    outs = W.grad_lap_outputs(3)
+    g = torch.tensor(rng.standard_normal((len(outs), pos.shape[0])), device="cuda")
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    plan = DcpsePlan(3, outs, stream=a)
+    plan.build_neighbors(p, 2.8 * h)
+    plan.assemble(p, FAST64)
+    w = [plan.output_weights(o)[0] for o in range(len(outs))]
+    ref, grad = [x.clone() for x in w], plan.vjp_positions(p, f, g)
+    torch.cuda.synchronize()
+    for spin in (SPIN, 0):
+        for x in w:
+            x.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(a):
+            torch.cuda._sleep(spin)
+        plan.set_stream(a)
+        plan.assemble(p, FAST64 | C.ASSEMBLE_ASYNC)
+        plan.set_stream(b)
+        got = plan.vjp_positions(p, f, g)
+        torch.cuda.synchronize()
+        assert torch.equal(got, grad)
+        assert all(torch.equal(x, r) for x, r in zip(w, ref))
+    plan.close()
