@@ -1194,7 +1194,7 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
         if (P->per[d] && cg.nc[d] < 5) packed = 0;
     if (!packed) cg = make_grid(rmax * (1.0 + 1e-9));
     const int64_t ncell = (int64_t)cg.nc[0] * cg.nc[1] * cg.nc[2];
-    int32_t *cell = nullptr, *ccount = nullptr, *cidx = nullptr, *counts = nullptr, *tmp = nullptr;
+    int32_t *cell = nullptr, *ccount = nullptr, *cidx = nullptr, *counts = nullptr, *tmp = nullptr, *left = nullptr;
     int64_t *cstart = nullptr, *fill = nullptr, *scan_tmp = nullptr;
     double* spos = nullptr;
     float4* srel = nullptr;
@@ -1206,6 +1206,7 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
         dfree(cidx);
         dfree(counts);
         dfree(tmp);
+        dfree(left);
         dfree(cstart);
         dfree(fill);
         dfree(scan_tmp);
@@ -1222,8 +1223,8 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
     if (e == cudaSuccess) e = dalloc(&scan_tmp, scan_tmp_elems(std::max<int64_t>(ncell, n)));
     if (e == cudaSuccess) e = dalloc(&spos, (size_t)ns * dim);
     if (e == cudaSuccess) e = dalloc(&srel, (size_t)std::max<int64_t>(ns, 1));
-    if (e == cudaSuccess) e = dalloc(&maxk, 1);
-    if (e == cudaSuccess) e = cudaMemsetAsync(maxk, 0, sizeof(int), s);
+    if (e == cudaSuccess) e = dalloc(&maxk, 2);  // longest row, particles left by the group search
+    if (e == cudaSuccess) e = cudaMemsetAsync(maxk, 0, 2 * sizeof(int), s);
     P->tstart(DCPSE_K_NEIGHBORS);
     if (e == cudaSuccess) e = build_cells(dim, ps, ns, cg, plan_geom(P), cell, ccount, cstart, fill, cidx, spos, srel, scan_tmp, s);
     NbrArgs a{};
@@ -1261,18 +1262,26 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
         for (int d = 0; d < dim; ++d) ball /= std::max(hi[d] - lo[d], rmax);
         const double want = 1.3 * ball * (double)n + 16.0;
         row_cap = want < 1024.0 ? ((int)want + 31) / 32 * 32 : 1024;  // (NaN, of an infinite cutoff: 1024)
-        if ((int64_t)row_cap * n * (int64_t)sizeof(int32_t) > kStageBytes || dalloc(&tmp, (size_t)row_cap * n) != cudaSuccess) {
+        if ((int64_t)row_cap * n * (int64_t)sizeof(int32_t) > kStageBytes || dalloc(&tmp, (size_t)row_cap * n) != cudaSuccess ||
+            dalloc(&left, (size_t)n) != cudaSuccess) {
             cudaGetLastError();
+            dfree(tmp);
             row_cap = 0;
         }
     }
-    if (e == cudaSuccess) e = row_cap > 0 ? stage_neighbors(a, counts, maxk, tmp, row_cap, s) : count_neighbors(a, counts, maxk, s);
-    if (e == cudaSuccess) e = exclusive_scan_i32(counts, n, P->rowptr, scan_tmp, s);
     int64_t nnz = 0;
-    int hk = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&nnz, P->rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&hk, maxk, sizeof(int), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    int found[2] = {0, 0};
+    auto offsets = [&](cudaError_t er) {
+        if (er == cudaSuccess) er = exclusive_scan_i32(counts, n, P->rowptr, scan_tmp, s);
+        if (er == cudaSuccess) er = cudaMemcpyAsync(&nnz, P->rowptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
+        if (er == cudaSuccess) er = cudaMemcpyAsync(found, maxk, sizeof found, cudaMemcpyDeviceToHost, s);
+        if (er == cudaSuccess) er = cudaStreamSynchronize(s);
+        return er;
+    };
+    if (e == cudaSuccess)
+        e = offsets(row_cap > 0 ? stage_neighbors(a, counts, maxk, tmp, row_cap, left, s) : count_neighbors(a, counts, maxk, s));
+    if (e == cudaSuccess && found[1] > 0) e = offsets(stage_left(a, counts, maxk, tmp, row_cap, left, found[1], s));
+    const int hk = found[0];
     if (hk > row_cap) {  // (no staging rows, or a row longer than them)
         dfree(tmp);
         row_cap = 0;

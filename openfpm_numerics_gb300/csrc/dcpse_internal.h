@@ -75,8 +75,13 @@ cudaError_t fill_neighbors(const NbrArgs& a, const int64_t* rowptr, int32_t* tmp
 // One search for counts and columns (one set on a packed grid, the domain set
 // being the support set): the neighbours of p, unsorted, to stage[p * cap ...],
 // the first cap of them; then sorted into cols, when no row is longer than cap.
+// d_maxk[1] particles (zeroed by the caller), in left[n_dom], stay to be searched
+// by stage_left: those of groups too crowded for one warp.
 bool stage_neighbors_serves(const NbrArgs& a);
-cudaError_t stage_neighbors(const NbrArgs& a, int32_t* counts, int* d_maxk, int32_t* stage, int cap, cudaStream_t s);
+cudaError_t stage_neighbors(const NbrArgs& a, int32_t* counts, int* d_maxk, int32_t* stage, int cap, int32_t* left,
+                            cudaStream_t s);
+cudaError_t stage_left(const NbrArgs& a, int32_t* counts, int* d_maxk, int32_t* stage, int cap, const int32_t* left,
+                       int nleft, cudaStream_t s);
 cudaError_t sort_staged(const NbrArgs& a, const int64_t* rowptr, const int32_t* stage, int cap, int32_t* cols,
                         cudaStream_t s);
 

@@ -21,6 +21,18 @@
 // the FP64 predicate within the margin and for NaN.
 #pragma once
 
+// Most steps of one warp, particles x chunks of 32 U candidates; the particles of
+// a group beyond it go to the warp-per-particle search (stage_left).  Cells take
+// half the largest radius as their side, so a group of a part whose own radii are
+// r times smaller holds r^2 (2D) or r^3 times the particles and as many times the
+// candidates, all for one warp: 2e5 points in 2D, 30 % of them in a patch of
+// radii 8 times smaller, took 72 ms without a bound, 3.4 ms with one (5.3 ms by
+// two passes of a warp per particle).  Ordinary groups take about 110 steps, those
+// of a part with half the radii 1,500.  Between 512 and 8192, 1024 was fastest or
+// within 2 % of it on nearly all of 33 sets (1 to 8 times smaller radii, clusters,
+// grids of few cells): that part at 2e5 points 0.94 ms with 2048, 0.64 with 1024.
+constexpr int64_t kGroupSteps = 1024;
+
 struct GroupGrid {
     int ng[3];       // groups per axis
     int64_t total;
@@ -28,7 +40,8 @@ struct GroupGrid {
 
 template <int DIM, int G, int U>
 __global__ void __launch_bounds__(256) nbr_group_kernel(NbrArgs a, GroupGrid gg, int32_t* __restrict__ counts,
-                                                        int* maxk, int32_t* __restrict__ stage, int cap) {
+                                                        int* maxk, int32_t* __restrict__ stage, int cap,
+                                                        int32_t* __restrict__ left) {
     constexpr int W = G + 2 * kPackR;                 // cells of the region per axis
     constexpr int NR = DIM == 3 ? W * W : W;          // its rows along axis 0
     constexpr int NS = 2 * NR;                        // segments: a row, and its part wrapped around axis 0
@@ -109,6 +122,18 @@ __global__ void __launch_bounds__(256) nbr_group_kernel(NbrArgs a, GroupGrid gg,
             total += __shfl_sync(full, e, 31);
         }
         __syncwarp();
+        if ((int64_t)np * ((total + 32 * U - 1) / (32 * U)) > kGroupSteps) {
+            // a crowd: its particles to the warp-per-particle search
+            int at = lane == 0 ? atomicAdd(&maxk[1], np) : 0;
+            at = __shfl_sync(full, at, 0);
+            for (int r = 0; r < PR; ++r) {
+                const int t0 = __shfl_sync(full, pstart, r), len = __shfl_sync(full, plen, r);
+                for (int i = lane; i < len; i += 32) left[at + i] = a.cidx[t0 + i];
+                at += len;
+            }
+            __syncwarp();  // the next group rewrites the segments
+            continue;
+        }
         for (int p0 = 0; p0 < np; p0 += 32) {
             const int nb = min(32, np - p0);
             // lane i's particle
@@ -254,7 +279,8 @@ inline int group_side(const NbrArgs& a) {
 }
 
 template <int DIM, int G, int U>
-cudaError_t launch_group(const NbrArgs& a, int32_t* counts, int* maxk, int32_t* stage, int cap, cudaStream_t s) {
+cudaError_t launch_group(const NbrArgs& a, int32_t* counts, int* maxk, int32_t* stage, int cap, int32_t* left,
+                         cudaStream_t s) {
     GroupGrid gg{};
     gg.total = 1;
     for (int d = 0; d < 3; ++d) {
@@ -263,6 +289,6 @@ cudaError_t launch_group(const NbrArgs& a, int32_t* counts, int* maxk, int32_t* 
     }
     const int64_t blocks = (gg.total + 7) / 8;
     nbr_group_kernel<DIM, G, U><<<(unsigned)std::min<int64_t>(blocks, 0x7fffffff), 256, 0, s>>>(a, gg, counts, maxk,
-                                                                                              stage, cap);
+                                                                                              stage, cap, left);
     return cudaGetLastError();
 }

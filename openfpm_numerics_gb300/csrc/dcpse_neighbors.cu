@@ -472,23 +472,35 @@ __device__ __forceinline__ int pack_cell(int c, int t, int nc, int per) {
     return v;
 }
 
-template <int DIM, bool FILL>
+// kCount: counts and *maxk.  kFill: the columns to tmp at rowptr.  kStage: both, of
+// the particles list[0 .. nlist), the columns to their staging rows of cap entries
+// in tmp.
+enum PackMode { kCount, kFill, kStage };
+
+template <int DIM, PackMode MODE>
 __global__ void __launch_bounds__(256) nbr_packed_kernel(NbrArgs a, int32_t* __restrict__ counts, int* maxk,
                                                          const int64_t* __restrict__ rowptr,
-                                                         int32_t* __restrict__ tmp) {
+                                                         int32_t* __restrict__ tmp, const int32_t* __restrict__ list,
+                                                         int nlist, int row_cap) {
+    constexpr bool FILL = MODE != kCount;
     const int lane = threadIdx.x & 31;
     const int64_t warp0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const unsigned lt_mask = (1u << lane) - 1u;
     const unsigned full = 0xffffffffu;
     constexpr int NR = DIM == 3 ? kPackW * kPackW : (DIM == 2 ? kPackW : 1);  // stencil rows
-    for (int64_t pb = warp0 * 32; pb < a.n_dom; pb += nwarps * 32) {
+    // particles a warp takes at a time (of a short list: fewer, so that every warp has some)
+    const int64_t np = MODE == kStage ? nlist : a.n_dom;
+    const int take = MODE == kStage ? (int)min((int64_t)32, max((int64_t)1, np / nwarps)) : 32;
+    for (int64_t pb = warp0 * take; pb < np; pb += nwarps * take) {
+        int listed = 0;
         float tin = 0.f, tout = 0.f;
         PackStencil S;
         {
             double x[3] = {0.0, 0.0, 0.0};
-            const int64_t pl = pb + lane;
-            if (pl < a.n_dom) {
+            int64_t pl = pb + lane;
+            if (pl < np && lane < take) {
+                if (MODE == kStage) pl = listed = list[pl];
 #pragma unroll
                 for (int d = 0; d < DIM; ++d) x[d] = a.pd[pl * DIM + d];
                 const double rc = a.rcut_pp ? a.rcut_pp[pl] : a.rcut;
@@ -498,9 +510,9 @@ __global__ void __launch_bounds__(256) nbr_packed_kernel(NbrArgs a, int32_t* __r
             }
             make_pack_stencil<DIM>(a, x, S);
         }
-        const int nb = (int)min((int64_t)32, a.n_dom - pb);
+        const int nb = (int)min((int64_t)take, np - pb);
         for (int i = 0; i < nb; ++i) {
-            const int64_t p = pb + i;
+            const int64_t p = MODE == kStage ? (int64_t)__shfl_sync(full, listed, i) : pb + i;
             const float ptin = __shfl_sync(full, tin, i), ptout = __shfl_sync(full, tout, i);
             const unsigned valid = __shfl_sync(full, S.valid, i), fastm = __shfl_sync(full, S.fast, i);
             const bool xwrap = __shfl_sync(full, (int)S.xwrap, i) != 0;
@@ -511,8 +523,9 @@ __global__ void __launch_bounds__(256) nbr_packed_kernel(NbrArgs a, int32_t* __r
                 pc[d] = __shfl_sync(full, S.c[d], i);
                 prc[d] = __shfl_sync(full, S.rpc[d], i);
             }
-            const int64_t base = FILL ? rowptr[p] : 0;
-            const int64_t cap = FILL ? rowptr[p + 1] - base : 0;  // the count pass's result
+            const int64_t base = MODE == kStage ? p * row_cap : (FILL ? rowptr[p] : 0);
+            // (the count pass's result)
+            const int64_t cap = MODE == kStage ? row_cap : (FILL ? rowptr[p + 1] - base : 0);
             int k = 0;
             // classifies candidate t (valid when has) of the cell-ordered
             // support; r0..r2 = x_p - corner of its cell, fast = FP32 allowed
@@ -637,7 +650,7 @@ __global__ void __launch_bounds__(256) nbr_packed_kernel(NbrArgs a, int32_t* __r
                     }
                 }
             }
-            if (!FILL && lane == 0) {
+            if (MODE != kFill && lane == 0) {
                 counts[p] = k;
                 atomicMax(maxk, k);
             }
@@ -918,9 +931,9 @@ cudaError_t count_neighbors(const NbrArgs& a, int32_t* counts, int* d_maxk, cuda
     if (a.n_dom == 0) return cudaSuccess;
     int grid = grid_for(a.n_dom * 32, 256);
     if (a.packed) {
-        if (a.dim == 1) nbr_packed_kernel<1, false><<<grid, 256, 0, s>>>(a, counts, d_maxk, nullptr, nullptr);
-        else if (a.dim == 2) nbr_packed_kernel<2, false><<<grid, 256, 0, s>>>(a, counts, d_maxk, nullptr, nullptr);
-        else nbr_packed_kernel<3, false><<<grid, 256, 0, s>>>(a, counts, d_maxk, nullptr, nullptr);
+        if (a.dim == 1) nbr_packed_kernel<1, kCount><<<grid, 256, 0, s>>>(a, counts, d_maxk, nullptr, nullptr, nullptr, 0, 0);
+        else if (a.dim == 2) nbr_packed_kernel<2, kCount><<<grid, 256, 0, s>>>(a, counts, d_maxk, nullptr, nullptr, nullptr, 0, 0);
+        else nbr_packed_kernel<3, kCount><<<grid, 256, 0, s>>>(a, counts, d_maxk, nullptr, nullptr, nullptr, 0, 0);
         return cudaGetLastError();
     }
     if (a.dim == 1) nbr_kernel<1, false><<<grid, 256, 0, s>>>(a, counts, d_maxk, nullptr, nullptr);
@@ -931,15 +944,27 @@ cudaError_t count_neighbors(const NbrArgs& a, int32_t* counts, int* d_maxk, cuda
 
 bool stage_neighbors_serves(const NbrArgs& a) { return group_side(a) > 0; }
 
-cudaError_t stage_neighbors(const NbrArgs& a, int32_t* counts, int* d_maxk, int32_t* stage, int cap, cudaStream_t s) {
+cudaError_t stage_neighbors(const NbrArgs& a, int32_t* counts, int* d_maxk, int32_t* stage, int cap, int32_t* left,
+                            cudaStream_t s) {
     if (a.n_dom == 0) return cudaSuccess;
     const int G = group_side(a);
     if (a.dim == 3)
-        return G == 2 ? launch_group<3, 2, 4>(a, counts, d_maxk, stage, cap, s)
-                      : launch_group<3, 1, 4>(a, counts, d_maxk, stage, cap, s);
-    if (G == 4) return launch_group<2, 4, 2>(a, counts, d_maxk, stage, cap, s);
-    return G == 2 ? launch_group<2, 2, 2>(a, counts, d_maxk, stage, cap, s)
-                  : launch_group<2, 1, 2>(a, counts, d_maxk, stage, cap, s);
+        return G == 2 ? launch_group<3, 2, 4>(a, counts, d_maxk, stage, cap, left, s)
+                      : launch_group<3, 1, 4>(a, counts, d_maxk, stage, cap, left, s);
+    if (G == 4) return launch_group<2, 4, 2>(a, counts, d_maxk, stage, cap, left, s);
+    return G == 2 ? launch_group<2, 2, 2>(a, counts, d_maxk, stage, cap, left, s)
+                  : launch_group<2, 1, 2>(a, counts, d_maxk, stage, cap, left, s);
+}
+
+cudaError_t stage_left(const NbrArgs& a, int32_t* counts, int* d_maxk, int32_t* stage, int cap, const int32_t* left,
+                       int nleft, cudaStream_t s) {
+    if (nleft <= 0) return cudaSuccess;
+    const int grid = grid_for((int64_t)nleft * 32, 256);
+    if (a.dim == 3)
+        nbr_packed_kernel<3, kStage><<<grid, 256, 0, s>>>(a, counts, d_maxk, nullptr, stage, left, nleft, cap);
+    else
+        nbr_packed_kernel<2, kStage><<<grid, 256, 0, s>>>(a, counts, d_maxk, nullptr, stage, left, nleft, cap);
+    return cudaGetLastError();
 }
 
 cudaError_t sort_staged(const NbrArgs& a, const int64_t* rowptr, const int32_t* stage, int cap, int32_t* cols,
@@ -953,9 +978,9 @@ cudaError_t fill_neighbors(const NbrArgs& a, const int64_t* rowptr, int32_t* tmp
     if (a.n_dom == 0) return cudaSuccess;
     int grid = grid_for(a.n_dom * 32, 256);
     if (a.packed) {
-        if (a.dim == 1) nbr_packed_kernel<1, true><<<grid, 256, 0, s>>>(a, nullptr, nullptr, rowptr, tmp);
-        else if (a.dim == 2) nbr_packed_kernel<2, true><<<grid, 256, 0, s>>>(a, nullptr, nullptr, rowptr, tmp);
-        else nbr_packed_kernel<3, true><<<grid, 256, 0, s>>>(a, nullptr, nullptr, rowptr, tmp);
+        if (a.dim == 1) nbr_packed_kernel<1, kFill><<<grid, 256, 0, s>>>(a, nullptr, nullptr, rowptr, tmp, nullptr, 0, 0);
+        else if (a.dim == 2) nbr_packed_kernel<2, kFill><<<grid, 256, 0, s>>>(a, nullptr, nullptr, rowptr, tmp, nullptr, 0, 0);
+        else nbr_packed_kernel<3, kFill><<<grid, 256, 0, s>>>(a, nullptr, nullptr, rowptr, tmp, nullptr, 0, 0);
     } else if (a.dim == 1) {
         nbr_kernel<1, true><<<grid, 256, 0, s>>>(a, nullptr, nullptr, rowptr, tmp);
     } else if (a.dim == 2) {

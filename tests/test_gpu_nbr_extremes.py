@@ -33,3 +33,46 @@ def test_cutoffs_beyond_the_set(cuda, dim, rcut):
     every = np.arange(n)
     assert np.array_equal(rp, np.arange(n + 1) * (n - 1))
     assert np.array_equal(cols.reshape(n, n - 1), np.array([np.delete(every, p) for p in range(n)]))
+
+
+def _patch(n, dim, ratio, share, seed):
+    """n points, `share` of them in a patch whose spacing is `ratio` times
+    smaller, each with a radius of about 30 (2D) or 90 neighbours."""
+    rng = np.random.default_rng(seed)
+    nd = int(n * share)
+    h = (1.0 / (n - nd)) ** (1.0 / dim)
+    side = nd ** (1.0 / dim) * h / ratio
+    wide, dense = rng.random((n - nd, dim)), 0.6 - side / 2 + side * rng.random((nd, dim))
+    rc = (3.1 if dim == 2 else 2.8) * h
+    near = np.all(np.abs(wide - 0.6) < side / 2, axis=1)
+    radii = np.concatenate([np.where(near, rc / ratio, rc), np.full(nd, rc / ratio)])
+    order = rng.permutation(n)
+    return np.vstack([wide, dense])[order], radii[order]
+
+
+@pytest.mark.parametrize("dim,n,ratio,share", [(2, 6000, 4, 0.1), (2, 6000, 8, 0.3), (3, 6000, 3, 0.3), (3, 4000, 4, 0.5)])
+@pytest.mark.parametrize("periodic", [False, True])
+def test_crowded_groups(cuda, orc, dim, n, ratio, share, periodic):
+    """Groups of cells too crowded for one warp, beside ordinary ones; the longest
+    rows are longer than the staging rows in some of these sets."""
+    pos, radii = _patch(n, dim, ratio, share, 72)
+    if periodic:  # (the patch across the box's faces)
+        pos = np.mod(pos + 0.4, 1.0)
+    box = ((0.0,) * dim, (1.0,) * dim, (1,) * dim) if periodic else None
+    for self_skip in (True, False):
+        rp, cols = _build(pos, 0.0, box, radii, self_skip)
+        erp, ecols = orc.neighbors(pos, 0.0, rcut_pp=radii, box=box, self_skip=self_skip)
+        assert np.array_equal(rp, erp) and np.array_equal(cols, ecols)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_crowds_of_long_rows(cuda, orc, dim):
+    """A cluster under one cutoff: rows longer than the staging rows, found by both
+    searches of one build."""
+    rng = np.random.default_rng(73)
+    pos = np.vstack([rng.random((4000, dim)), 0.45 + 0.1 * rng.random((3000, dim))])
+    rcut = 2.5 * 7000 ** (-1.0 / dim)
+    rp, cols = _build(pos, rcut)
+    erp, ecols = orc.neighbors(pos, rcut)
+    assert np.diff(erp).max() > 300
+    assert np.array_equal(rp, erp) and np.array_equal(cols, ecols)
