@@ -171,6 +171,8 @@ constexpr int64_t kStageBytes = int64_t(8) << 30;
 // Largest scratch of one assembly batch; larger clouds are assembled in
 // batches of particles (the result does not depend on the batch size).
 constexpr int64_t kAsmScratchBytes = int64_t(512) << 20;
+// particles of the smallest batches, where device memory is short (a megabyte or two)
+constexpr int64_t kAsmBatchLeast = 256;
 
 struct CudaRt {
     typedef cudaError_t Error;
@@ -1092,14 +1094,15 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
     dfree(P->cell_order);
     P->list_version++;
     dfree(P->cols);
-    if (int rc = settle()) return rc;
-    P->n = n;
+    P->n = -1;  // no list until it is built
     P->nnz = 0;
     P->maxk = 0;
+    if (int rc = settle()) return rc;
     DCPSE_CK(dalloc(&P->rowptr, (size_t)n + 1));
     if (n == 0) {
         DCPSE_CK(cudaMemsetAsync(P->rowptr, 0, sizeof(int64_t), s));
         DCPSE_CK(dalloc(&P->cols, kPad));
+        P->n = 0;
         return DCPSE_OK;
     }
     // the support set: the domain set itself, a second set, or (surface
@@ -1282,12 +1285,19 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
         e = offsets(row_cap > 0 ? stage_neighbors(a, counts, maxk, tmp, row_cap, left, s) : count_neighbors(a, counts, maxk, s));
     if (e == cudaSuccess && found[1] > 0) e = offsets(stage_left(a, counts, maxk, tmp, row_cap, left, found[1], s));
     const int hk = found[0];
-    if (hk > row_cap) {  // (no staging rows, or a row longer than them)
+    auto drop_staging = [&] {
+        const bool had = tmp != nullptr;
         dfree(tmp);
+        dfree(left);
         row_cap = 0;
-    }
+        return had;
+    };
+    if (hk > row_cap) drop_staging();  // (no staging rows, or a row longer than them)
+    // the columns, if need be in the staging rows' place: the fill pass then finds
+    // them again
+    if (e == cudaSuccess)
+        e = with_room<CudaRt>([&] { return dalloc(&P->cols, (size_t)nnz + kPad); }, drop_staging);
     if (e == cudaSuccess && row_cap == 0) e = dalloc(&tmp, nnz);
-    if (e == cudaSuccess) e = dalloc(&P->cols, nnz + kPad);
     if (e == cudaSuccess)
         e = row_cap > 0 ? sort_staged(a, P->rowptr, tmp, row_cap, P->cols, s) : fill_neighbors(a, P->rowptr, tmp, P->cols, s);
     P->tstop(DCPSE_K_NEIGHBORS);
@@ -1298,9 +1308,12 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
         // the particles' renumbering order (one set; P->reorder_order): the
         // apply's sliced layout may renumber rows and columns by it (the
         // cells' own order, if the order's work space cannot be had)
-        ez = dalloc(&key, (size_t)std::max<int64_t>(ns, 1));
-        if (ez == cudaSuccess) ez = dalloc(&zord, (size_t)std::max<int64_t>(ns, 1));
-        if (ez == cudaSuccess) ez = dalloc(&ztmp, (size_t)order_tmp_elems(dim, ns, cg, P->reorder_order));
+        auto get = [&](auto** p, int64_t count) {
+            return with_room<CudaRt>([&] { return dalloc(p, (size_t)std::max<int64_t>(count, 1)); }, drop_staging);
+        };
+        ez = get(&key, ns);
+        if (ez == cudaSuccess) ez = get(&zord, ns);
+        if (ez == cudaSuccess) ez = get(&ztmp, order_tmp_elems(dim, ns, cg, P->reorder_order));
         if (ez == cudaSuccess) ez = particle_order(dim, ps, cell, ns, cg, P->reorder_order, key, ztmp, zord, s);
         if (ez != cudaSuccess) cudaGetLastError();
     }
@@ -1318,6 +1331,7 @@ int dcpse_build_neighbors(dcpse_plan_t* P, const double* d_pos, int64_t n, doubl
     dfree(zord);
     cleanup();
     if (e != cudaSuccess) return fail(DCPSE_ERR_CUDA, std::string("neighbour build: ") + cudaGetErrorString(e));
+    P->n = n;
     P->nnz = nnz;
     P->maxk = hk;
     P->surf_pending = P->surface();
@@ -1335,9 +1349,9 @@ int dcpse_set_neighbors(dcpse_plan_t* P, int64_t n, int64_t nnz, const int64_t* 
     dfree(P->cell_order);
     P->list_version++;
     dfree(P->cols);
+    P->n = -1;  // no list until it is checked
+    P->nnz = 0;
     if (int rc = settle()) return rc;
-    P->n = n;
-    P->nnz = nnz;
     DCPSE_CK(dalloc(&P->rowptr, (size_t)n + 1));
     DCPSE_CK(dalloc(&P->cols, nnz + kPad));
     DCPSE_CK(cudaMemcpyAsync(P->rowptr, d_rowptr, sizeof(int64_t) * (n + 1), cudaMemcpyDeviceToDevice, s));
@@ -1364,10 +1378,10 @@ int dcpse_set_neighbors(dcpse_plan_t* P, int64_t n, int64_t nnz, const int64_t* 
         dfree(P->rowptr);
         P->list_version++;
         dfree(P->cols);
-        P->n = -1;
-        P->nnz = 0;
         return fail(DCPSE_ERR_ARG, "invalid CSR neighbour list (row offsets or column indices)");
     }
+    P->n = n;
+    P->nnz = nnz;
     P->maxk = (int)(h[1] & 0xffffffffu);
     return DCPSE_OK;
 }
@@ -1388,24 +1402,21 @@ int ensure_sell64(dcpse_plan_t* P);
 // kAsmScratchBytes (the Gram entries, coefficients and scaled offsets of the
 // particles in flight); smaller batches where device memory is short (the
 // result does not depend on the batch size).
-int batch_scratch(double*& scratch, int64_t& have, AsmArgs& a, int64_t per) {
+extern "C++" template <class Room>
+int batch_scratch(double*& scratch, int64_t& have, AsmArgs& a, int64_t per, Room room) {
     int64_t nb = std::min<int64_t>(a.n, std::max<int64_t>(4096, kAsmScratchBytes / per));
-    cudaError_t e = cudaSuccess;
-    while (have < nb * per + 16) {
-        const int64_t bytes = nb * per + 16;
+    if (have < nb * per + 16) {
         dfree(scratch);
         have = 0;
-        e = dalloc(&scratch, (size_t)(bytes + 7) / 8);
-        if (e == cudaSuccess) {
-            have = bytes;
-        } else if (e == cudaErrorMemoryAllocation && nb > 4096) {
+        auto alloc = [&](int64_t m) { return dalloc(&scratch, (size_t)(m * per + 16 + 7) / 8); };
+        cudaError_t e = with_room<CudaRt>([&] { return alloc(nb); }, room);
+        if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError();
-            nb = std::max<int64_t>(4096, nb / 2);
-        } else {
-            break;
+            e = with_less<CudaRt>(nb, std::min<int64_t>(nb, kAsmBatchLeast), alloc);
         }
+        DCPSE_CK(e);
+        have = nb * per + 16;
     }
-    DCPSE_CK(e);
     a.scratch = scratch;
     a.scratch_particles = nb;
     return DCPSE_OK;
@@ -1451,12 +1462,20 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
     dfree(P->rowsum);
     P->rowsum_prec = -1;
     P->free_vsell_weights();
-    if ((flags & DCPSE_STORE_OUT_F32) && !P->w32) DCPSE_CK(dalloc(&P->w32, (size_t)P->nout * nnz + kPad));
+    // (the sliced copy that is kept is given up where memory is short)
+    auto spares = [&] {
+        const bool had = P->sell_row != nullptr;
+        P->free_sell();
+        return had;
+    };
+    auto get = [&](auto** p, size_t count) { return with_room<CudaRt>([&] { return dalloc(p, count); }, spares); };
+    const size_t nw = (size_t)P->nout * nnz + kPad;
+    if ((flags & DCPSE_STORE_OUT_F32) && !P->w32) DCPSE_CK(get(&P->w32, nw));
     if (!(flags & DCPSE_STORE_OUT_F32)) dfree(P->w32);
     if ((flags & DCPSE_STORE_OUT_F32_RESID) && !P->r16)
-        DCPSE_CK(dalloc_bytes(&P->r16, ((size_t)P->nout * nnz + kPad) * 2));
+        DCPSE_CK(with_room<CudaRt>([&] { return dalloc_bytes(&P->r16, nw * 2); }, spares));
     if (!(flags & DCPSE_STORE_OUT_F32_RESID)) dfree(P->r16);
-    if ((flags & DCPSE_STORE_OUT_F32_CORR) && !P->r32) DCPSE_CK(dalloc(&P->r32, (size_t)P->nout * nnz + kPad));
+    if ((flags & DCPSE_STORE_OUT_F32_CORR) && !P->r32) DCPSE_CK(get(&P->r32, nw));
     if (!(flags & DCPSE_STORE_OUT_F32_CORR)) dfree(P->r32);
     // not while an apply on the plan's previous stream still reads them, either
     if (t_given_up != given_up || (P->stream_changed && !capturing(s)))
@@ -1489,13 +1508,14 @@ int dcpse_assemble(dcpse_plan_t* P, const double* d_pos, const double* d_eps_fix
     a.err = P->d_err;
     a.order = nullptr;
     if (n > 0) {
-        if (int rc = batch_scratch(P->asm_scratch, P->asm_scratch_bytes, a, assembly_scratch_bytes(*P->htab, flags, P->maxk)))
+        if (int rc = batch_scratch(P->asm_scratch, P->asm_scratch_bytes, a,
+                                   assembly_scratch_bytes(*P->htab, flags, P->maxk), spares))
             return rc;
         const int64_t qb = assembly_qr_ws_bytes(*P->htab, flags);
         if (qb > 0 && P->qr_ws_bytes < qb) {
             dfree(P->qr_ws);
             P->qr_ws_bytes = 0;
-            DCPSE_CK(dalloc(&P->qr_ws, (size_t)(qb + 7) / 8));
+            DCPSE_CK(get(&P->qr_ws, (size_t)(qb + 7) / 8));
             P->qr_ws_bytes = qb;
         }
         a.qws = qb > 0 ? P->qr_ws : nullptr;
@@ -1829,7 +1849,8 @@ int dcpse_vjp_positions(dcpse_plan_t* P, const double* d_pos, const double* d_ep
         a.scratch = P->vjp_scratch;
         a.scratch_particles = P->vjp_batch;
     } else {
-        if (int rc = batch_scratch(P->vjp_scratch, P->vjp_scratch_bytes, a, vjp_scratch_bytes(*P->htab, P->maxk)))
+        if (int rc = batch_scratch(P->vjp_scratch, P->vjp_scratch_bytes, a, vjp_scratch_bytes(*P->htab, P->maxk),
+                                   [] { return false; }))
             return rc;
         P->vjp_batch = a.scratch_particles;
     }
@@ -1949,7 +1970,12 @@ int dcpse_rk4_gs_adjoint_prepare(dcpse_plan_t* P, int precision) {
                                   total, P->tsell_cols, nullptr, nullptr, P->stream);
                 if (e == cudaSuccess)
                     e = narrow_columns(P->tsell_row, P->tsell_off, P->tsell_cols, total, ns, 1, P->tsell_narrow, P->stream);
-                if (e == cudaSuccess) e = dalloc(&P->tsell_w, (size_t)total + kPad);
+                if (e == cudaSuccess)
+                    e = with_room<CudaRt>([&] { return dalloc(&P->tsell_w, (size_t)total + kPad); }, [&] {
+                        const bool had = P->tsell_narrow.d != nullptr;
+                        dcpse_plan_s::free_narrow(P->tsell_narrow);
+                        return had;
+                    });
             }
             if (e == cudaSuccess)
                 e = sell_fill(P->t_row, P->t_src, P->wT32, nullptr, P->nnz, 1, P->n, 1, P->tsell_row, P->tsell_off,
@@ -2253,7 +2279,12 @@ cudaError_t spare_or(T*& live, T*& spare, size_t count) {
 // absent (the CSR kernels serve), other errors fail.
 extern "C++" template <typename Alloc, typename Fill, typename Release>
 int sell_stream(dcpse_plan_t* P, const char* what, Alloc alloc, Fill fill, Release release) {
-    cudaError_t e = alloc();
+    // (rather without the 16-bit columns than without the weights)
+    cudaError_t e = with_room<CudaRt>(alloc, [&] {
+        const bool had = P->sell_narrow.d != nullptr;
+        dcpse_plan_s::free_narrow(P->sell_narrow);
+        return had;
+    });
     if (e == cudaSuccess) e = fill();
     if (e == cudaSuccess) e = cudaStreamSynchronize(P->stream);
     if (e == cudaSuccess) return DCPSE_OK;

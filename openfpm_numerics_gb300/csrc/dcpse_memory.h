@@ -180,4 +180,27 @@ private:
     int plans_ = 0;
 };
 
+// alloc(), and where memory is short once more after room() has given something up
+// (it returns whether it had anything)
+template <class Rt, class Alloc, class Room>
+typename Rt::Error with_room(Alloc alloc, Room room) {
+    typename Rt::Error e = alloc();
+    if (e == Rt::no_memory && room()) {
+        Rt::clear_error();
+        e = alloc();
+    }
+    return e;
+}
+
+// alloc(count), with count halved (down to `least`) while memory is short
+template <class Rt, class Int, class Alloc>
+typename Rt::Error with_less(Int& count, Int least, Alloc alloc) {
+    for (;;) {
+        const typename Rt::Error e = alloc(count);
+        if (e != Rt::no_memory || count <= least) return e;
+        Rt::clear_error();
+        count = std::max(least, count / 2);
+    }
+}
+
 }  // namespace dcpse

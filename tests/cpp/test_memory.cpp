@@ -128,6 +128,40 @@ int main() {
         CHECK(Fake::used == 0);
     }
     {
+        // short of memory: a second try after something was given up, then less
+        Pool pool;
+        void *big, *p;
+        Fake::limit = Fake::used + (size_t(1) << 20);
+        CHECK(pool.alloc(&big, 900000) == 0);
+        auto room = [&] {
+            const bool had = big != nullptr;
+            pool.free(big);
+            big = nullptr;
+            return had;
+        };
+        auto want = [&] { return pool.alloc(&p, 600000); };
+        CHECK(dcpse::with_room<Fake>(want, room) == 0 && !big && p && Fake::last_error == 0);
+        pool.free(p);
+        Fake::limit = Fake::used;  // (the free block of 600,000 alone)
+        auto more = [&] { return pool.alloc(&p, 2000000); };
+        CHECK(dcpse::with_room<Fake>(more, room) == Fake::no_memory && !p);
+        Fake::clear_error();
+        Fake::limit = Fake::used + (size_t(1) << 20);
+        for (long least : {1L, 100L, 3000L}) {
+            long count = 4096;
+            const int e = dcpse::with_less<Fake>(count, least, [&](long c) { return pool.alloc(&p, (size_t)c * 4000); });
+            if (least == 3000) {
+                CHECK(e == Fake::no_memory && count == 3000);
+                Fake::clear_error();
+            } else {
+                CHECK(e == 0 && count == 256 && Fake::last_error == 0);
+                pool.free(p);
+            }
+        }
+        pool.release();
+        Fake::limit = ~size_t(0) / 2;
+    }
+    {
         // threads: no two owners of a block at a time
         Pool pool;
         std::mutex m;

@@ -76,3 +76,27 @@ def test_crowds_of_long_rows(cuda, orc, dim):
     erp, ecols = orc.neighbors(pos, rcut)
     assert np.diff(erp).max() > 300
     assert np.array_equal(rp, erp) and np.array_equal(cols, ecols)
+
+
+def test_a_refused_build_leaves_no_list(cuda):
+    """After positions or a list that are refused the plan has no list: calls that
+    need one say so (they would read arrays that were never filled)."""
+    from openfpm_numerics_gb300 import _capi as C
+
+    pos = torch.tensor(W.lattice(12, 2)[0], device="cuda")
+    bad = pos.clone()
+    bad[3, 0] = float("inf")
+    plan = DcpsePlan(2, [[(1, 0)]])
+    rp = torch.arange(145, dtype=torch.int64, device="cuda")
+    for refused in (lambda: plan.build_neighbors(bad, 0.3),
+                    lambda: plan.set_neighbors(rp, torch.full((144,), 144, device="cuda"))):
+        plan.build_neighbors(pos, 0.3)
+        with pytest.raises(C.DcpseError):
+            refused()
+        assert plan.info()["n"] == -1
+        with pytest.raises(C.DcpseError) as e:
+            plan.assemble(pos, C.ASSEMBLE_FAST | C.STORE_OUT_F64)
+        assert e.value.code == C.ERR_STATE
+    plan.build_neighbors(pos, 0.3)
+    plan.assemble(pos, C.ASSEMBLE_FAST | C.STORE_OUT_F64)
+    plan.close()
