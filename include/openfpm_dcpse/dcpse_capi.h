@@ -99,6 +99,11 @@ int dcpse_version(void);
 int dcpse_plan_create(dcpse_plan_t** plan, int dim, int n_outputs, const int* terms_per_output,
                       const unsigned* signatures, unsigned order, double h_over_eps);
 int dcpse_plan_destroy(dcpse_plan_t* plan);
+/* Gives the device memory that released buffers of the plans still hold (at most
+ * 4 GiB, kept for re-use) back to the driver, as the end of the last plan and a
+ * failed allocation of the library do; for other users of the device.  Callable
+ * from any thread. */
+int dcpse_release_memory(void);
 /* stream: a cudaStream_t (NULL = legacy default stream) */
 int dcpse_plan_set_stream(dcpse_plan_t* plan, void* stream);
 /* Domain box and periodicity (minimum-image offsets along periodic axes).

@@ -17,6 +17,13 @@ from .operators import (  # noqa: F401
 )
 
 
+def release_memory():
+    """Give the device memory that closed plans' buffers still hold (at most
+    4 GiB, kept for re-use) back to the driver, e.g. when another allocator of
+    the process is short of it."""
+    _capi.call("dcpse_release_memory")
+
+
 def load():
     """Build (if needed) and load the CUDA extension; raises if unavailable."""
     return _capi.load()

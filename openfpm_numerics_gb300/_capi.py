@@ -29,6 +29,7 @@ SIGNATURES = {
     "dcpse_version": (_I, []),
     "dcpse_plan_create": (_I, [_PP, _I, _I, _PI, _PU, _c.c_uint, _D]),
     "dcpse_plan_destroy": (_I, [_P]),
+    "dcpse_release_memory": (_I, []),
     "dcpse_plan_set_stream": (_I, [_P, _P]),
     "dcpse_plan_set_box": (_I, [_P, _c.POINTER(_D), _c.POINTER(_D), _PI]),
     "dcpse_plan_set_support": (_I, [_P, _P, _I64, _I]),

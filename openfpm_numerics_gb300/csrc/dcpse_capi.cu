@@ -993,6 +993,11 @@ int dcpse_plan_destroy(dcpse_plan_t* P) {
     return DCPSE_OK;
 }
 
+int dcpse_release_memory(void) {
+    pool().release();
+    return DCPSE_OK;
+}
+
 int dcpse_plan_set_stream(dcpse_plan_t* P, void* stream) {
     if (int rc = check_plan(P)) return rc;
     if (P->stream != (cudaStream_t)stream) P->stream_changed = true;
@@ -2099,7 +2104,10 @@ int dcpse_rk4_gs_reverse_step(dcpse_plan_t* P, int precision, const void* const*
 int dcpse_device_alloc(void** ptr, uint64_t bytes) {
     if (!ptr) return fail(DCPSE_ERR_ARG, "NULL pointer");
     *ptr = nullptr;
-    DCPSE_CK(cudaMalloc(ptr, bytes ? bytes : 1));
+    DCPSE_CK(with_room<CudaRt>([&] { return cudaMalloc(ptr, bytes ? bytes : 1); }, [] {
+        pool().release();
+        return true;
+    }));
     return DCPSE_OK;
 }
 

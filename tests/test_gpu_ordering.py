@@ -233,3 +233,18 @@ def test_position_vjp_beside_a_pending_assembly(cuda):
         assert torch.equal(got, grad)
         assert all(torch.equal(x, r) for x, r in zip(w, ref))
     plan.close()
+
+
+def test_released_memory_can_be_given_back(cuda):
+    keep = DcpsePlan(2, [[(1, 0)]])
+    pos, h = W.lattice(48, 3, jitter=0.1, seed=86)
+    p = torch.tensor(pos, device="cuda")
+    plan = DcpsePlan(3, W.grad_lap_outputs(3))
+    plan.build_neighbors(p, 2.8 * h)
+    plan.assemble(p, FAST64)
+    plan.close()
+    torch.cuda.synchronize()
+    held = torch.cuda.mem_get_info()[0]
+    cuda.release_memory()
+    assert torch.cuda.mem_get_info()[0] - held > 200 << 20  # (the weights alone take 250 MB)
+    keep.close()
