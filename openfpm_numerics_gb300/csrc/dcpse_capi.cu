@@ -805,18 +805,31 @@ int fixed_into_plan(dcpse_plan_t* P, const double* d_f, const int32_t* inv) {
 // 16-bit columns of a sliced layout whose streams (columns and nout FP32 weight
 // streams) exceed L2; from L2 the columns' bytes do not matter and the list may
 // be applied only once.  Without room the 32-bit columns serve alone.
+// Only where three slices in four or more have them, and not on a renumbered
+// layout: the kernel that looks for them takes 64 registers to the plain one's 56
+// (measured with / without them, ms: shuffled 128^3 in the caller's numbering, no
+// slice, four outputs 0.816 / 0.790; 200^3 lattice, 88 % of them, 2.252 / 2.278;
+// renumbered 10^6 graded rows, 85 %, five outputs 0.170 / 0.157, one 0.086 / 0.082;
+// renumbered 128^3, 40 %, four outputs 0.667 / 0.671, one 0.312 / 0.309).
 constexpr int64_t kNarrowStreamBytes = int64_t(128) << 20;
+constexpr double kNarrowShare = 0.75;
 cudaError_t narrow_columns(const int32_t* srow, const int64_t* off, const int32_t* cols, int64_t total, int64_t nslices,
                            int nout, NarrowCols& nc, cudaStream_t s) {
     if (total * (4 + 4 * (int64_t)nout) <= kNarrowStreamBytes) return cudaSuccess;
+    unsigned long long *nfit = nullptr, fit = 0;
     if (dalloc(&nc.d, (size_t)total + kPad) != cudaSuccess ||
         dalloc(&nc.base, (size_t)narrow_bases(total, nslices)) != cudaSuccess ||
-        dalloc(&nc.flag, (size_t)nslices) != cudaSuccess) {
+        dalloc(&nc.flag, (size_t)nslices) != cudaSuccess || dalloc(&nfit, 1) != cudaSuccess) {
         cudaGetLastError();
         dcpse_plan_s::free_narrow(nc);
         return cudaSuccess;
     }
-    return sell_narrow(srow, off, cols, nslices, nc, s);
+    cudaError_t e = sell_narrow(srow, off, cols, nslices, nc, nfit, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&fit, nfit, sizeof fit, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    dfree(nfit);
+    if (e != cudaSuccess || (double)fit < kNarrowShare * (double)nslices) dcpse_plan_s::free_narrow(nc);
+    return e;
 }
 
 // SurfaceDcpse::accumulateAndDeleteNormalParticles on the plan's arrays: the
@@ -2250,7 +2263,7 @@ int ensure_sell_layout(dcpse_plan_t* P) {
         e = sell_fill(P->rowptr, P->cols, nullptr, nullptr, P->nnz, P->nout, P->n, P->two_set() ? 0 : 1,
                       P->sell_row, P->sell_off, total, P->sell_cols, nullptr, nullptr, P->stream, P->sell_perm,
                       P->sell_perm ? P->sell_inv : nullptr);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && !P->sell_perm)
         e = narrow_columns(P->sell_row, P->sell_off, P->sell_cols, total, ns, P->nout, P->sell_narrow, P->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(P->stream);
     if (e == cudaErrorMemoryAllocation) {

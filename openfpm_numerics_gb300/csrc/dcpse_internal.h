@@ -238,8 +238,9 @@ struct NarrowCols {
 };
 __host__ __device__ inline int64_t narrow_base(int64_t off, int64_t slice) { return off / 128 + slice; }
 inline int64_t narrow_bases(int64_t total, int64_t nslices) { return total / 128 + nslices + 1; }
+// *nfit: the slices with flag 1
 cudaError_t sell_narrow(const int32_t* srow, const int64_t* off, const int32_t* cols, int64_t nslices,
-                        const NarrowCols& nc, cudaStream_t s);
+                        const NarrowCols& nc, unsigned long long* nfit, cudaStream_t s);
 
 struct SellArgs {
     const int32_t* perm;   // position -> list row, or null (identity)

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) sell_fill_kernel(const int64_t* __restric
 __global__ void __launch_bounds__(256) sell_narrow_kernel(const int32_t* __restrict__ srow,
                                                           const int64_t* __restrict__ off,
                                                           const int32_t* __restrict__ cols, int64_t nslices,
-                                                          NarrowCols nc) {
+                                                          NarrowCols nc, unsigned long long* nfit) {
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s < nslices; s += nwarps) {
@@ -183,7 +183,10 @@ __global__ void __launch_bounds__(256) sell_narrow_kernel(const int32_t* __restr
                 if (j0 + u < L)
                     nc.d[b + (int64_t)(j0 + u) * kSlice + lane] = c[u] == row ? (uint16_t)0xffffu : (uint16_t)(c[u] - lo);
         }
-        if (lane == 0) nc.flag[s] = fits ? 1 : 0;
+        if (lane == 0) {
+            nc.flag[s] = fits ? 1 : 0;
+            if (fits) atomicAdd(nfit, 1ull);
+        }
     }
 }
 
@@ -682,10 +685,11 @@ cudaError_t sell_order(const int64_t* rowptr, int64_t n, int32_t* srow, int32_t*
 }
 
 cudaError_t sell_narrow(const int32_t* srow, const int64_t* off, const int32_t* cols, int64_t nslices,
-                        const NarrowCols& nc, cudaStream_t s) {
-    if (nslices == 0) return cudaSuccess;
+                        const NarrowCols& nc, unsigned long long* nfit, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(nfit, 0, sizeof *nfit, s);
+    if (e != cudaSuccess || nslices == 0) return e;
     const int grid = (int)std::min<int64_t>((nslices + 7) / 8, (int64_t)num_sms() * 8);
-    sell_narrow_kernel<<<grid, 256, 0, s>>>(srow, off, cols, nslices, nc);
+    sell_narrow_kernel<<<grid, 256, 0, s>>>(srow, off, cols, nslices, nc, nfit);
     return cudaGetLastError();
 }
 
