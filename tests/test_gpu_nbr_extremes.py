@@ -100,3 +100,31 @@ def test_a_refused_build_leaves_no_list(cuda):
     plan.build_neighbors(pos, 0.3)
     plan.assemble(pos, C.ASSEMBLE_FAST | C.STORE_OUT_F64)
     plan.close()
+
+
+@pytest.mark.parametrize("dim,cells", [(2, 30), (2, 100), (2, 160), (3, 8), (3, 24)])
+def test_outside_a_periodic_box(cuda, dim, cells):
+    """Particles just inside, just beyond and well outside a box with periodic
+    axes, in groups of one, two and four cells: the search by groups against the
+    two-pass search, which serves where the columns are a second set (here the
+    same positions)."""
+    rng = np.random.default_rng(74)
+    side = 1.0 / (cells + 0.5)
+    rcut = 2.0 * side
+    n = int((10 if dim == 2 else 2.5) * cells ** dim / (3.1 if dim == 2 else 1.0))
+    pos = rng.random((n, dim))
+    k = n // 8
+    edge = rng.integers(0, 2, (k, dim)).astype(float)
+    off = side * rng.choice([0.0, 1e-16, 1e-9, 1e-7, 9e-7, 1.1e-6, 1e-5, 0.3, 0.6, 3.0], (k, dim)) * rng.choice([-1, 1], (k, dim))
+    axes = rng.random((k, dim)) < 0.6
+    pos[:k] = np.where(axes, edge + off, pos[:k])
+    for per in ((1,) * dim, (0,) + (1,) * (dim - 1), (1,) + (0,) * (dim - 1)):
+        box = ((0.0,) * dim, (1.0,) * dim, per)
+        rp, cols = _build(pos, rcut, box, self_skip=False)
+        plan = DcpsePlan(dim, [[(1,) + (0,) * (dim - 1)]], box=box)
+        t = torch.tensor(pos, device="cuda")
+        plan.set_support(t.clone())
+        plan.build_neighbors(t, rcut)
+        rp2, cols2 = (x.cpu().numpy() for x in plan.neighbors())
+        plan.close()
+        assert np.array_equal(rp, rp2) and np.array_equal(cols, cols2)
