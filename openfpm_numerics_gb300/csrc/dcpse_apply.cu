@@ -65,7 +65,7 @@ __device__ __forceinline__ int64_t row_by_length(int64_t base, int64_t n, const 
 }
 
 // T terms of one sign, each D_t = sum_q (f_q + s f_p) K_t,pq in row order,
-// then their outputs' sums in term order: one sum f_q + s f_p per entry serves
+// then the output's sum in term order: one sum f_q + s f_p per entry serves
 // all terms, and the products run on the integer pipes, which leaves T + 1 FP64
 // operations per entry instead of 3 T.  FP64-pipe bound (82 % before its sums
 // became three-register dfmas); 96^3 Laplacian, three terms: 1.46 ms with a
@@ -80,9 +80,8 @@ struct TermsArgs {
     const int32_t* cols;
     const double* K[kTermsFused];
     const double* eip[kTermsFused];
-    double* out[kTermsFused];   // output of each term
-    unsigned fresh, last;       // bit t: term t begins / ends its output's terms in this launch
-    int accumulate;             // the first output continues an earlier launch
+    double* out;
+    int accumulate;             // the output continues an earlier launch
     double sign;
     const double* f;
 };
@@ -149,13 +148,11 @@ __global__ void __launch_bounds__(256) apply_terms_f64_kernel(TermsArgs a) {
             for (int u = 0; u < U; ++u) fq[u] = F.add(fq[u], fxp);
             add_products<T, U>(F, D, fq, k, len - j);
         }
-        double r = a.accumulate ? a.out[0][p] : 0.0;
+        double r = D[0] * a.eip[0][p];
+        if (a.accumulate) r = a.out[p] + r;
 #pragma unroll
-        for (int t = 0; t < T; ++t) {
-            const double v = D[t] * a.eip[t][p];
-            r = ((a.fresh >> t) & 1u) ? v : r + v;
-            if ((a.last >> t) & 1u) a.out[t][p] = r;
-        }
+        for (int t = 1; t < T; ++t) r = r + D[t] * a.eip[t][p];
+        a.out[p] = r;
     }
 }
 
@@ -639,10 +636,10 @@ cudaError_t launch_f64(int64_t n, int nout, const int64_t* rowptr, const int32_t
 
 }  // namespace
 
-// Terms of one output run (or several outputs), all of one sign, in plan order
-// (TermsArgs).  One launch for up to kTermsFused terms.
+// Terms of one output, all of one sign, in plan order (TermsArgs): up to
+// kTermsFused of them.
 cudaError_t apply_terms_f64(int64_t n, const int64_t* rowptr, const int32_t* cols, int nterms, const double* const* K,
-                            const double* const* eip, double* const* out, int accumulate, unsigned order,
+                            const double* const* eip, double* out, int accumulate, unsigned order,
                             const double* f, cudaStream_t s) {
     if (n == 0 || nterms == 0) return cudaSuccess;
     if (nterms > kTermsFused) return cudaErrorInvalidValue;
@@ -653,10 +650,8 @@ cudaError_t apply_terms_f64(int64_t n, const int64_t* rowptr, const int32_t* col
     for (int t = 0; t < nterms; ++t) {
         a.K[t] = K[t];
         a.eip[t] = eip[t];
-        a.out[t] = out[t];
-        if (t == 0 ? !accumulate : out[t] != out[t - 1]) a.fresh |= 1u << t;
-        if (t + 1 == nterms || out[t + 1] != out[t]) a.last |= 1u << t;
     }
+    a.out = out;
     a.accumulate = accumulate;
     a.sign = (order % 2 == 0) ? -1.0 : 1.0;
     a.f = f;

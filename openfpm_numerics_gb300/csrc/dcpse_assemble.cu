@@ -1023,11 +1023,12 @@ cudaError_t launch_qr(const AsmArgs& a, Split S, int64_t b0, int64_t nb, cudaStr
     S.pstride = qr_pstride(S, LPP);
     // without the table of Gram entries where it is what does not fit
     if (qr_bytes(S, LPP) > (size_t)smem_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, 227 * 1024)) S.qtab = 0;
-    if (S.qws) {
-        const int64_t grid = std::min<int64_t>((int64_t)num_sms() * kQrGlobalPerSm, nb);
-        qr_kernel<LPP, true><<<(unsigned)std::max<int64_t>(grid, 1), 32, 0, s>>>(a, S, b0, nb);
-        return cudaGetLastError();
-    }
+    if constexpr (LPP == 32)
+        if (S.qws) {
+            const int64_t grid = std::min<int64_t>((int64_t)num_sms() * kQrGlobalPerSm, nb);
+            qr_kernel<LPP, true><<<(unsigned)std::max<int64_t>(grid, 1), 32, 0, s>>>(a, S, b0, nb);
+            return cudaGetLastError();
+        }
     const size_t bytes = qr_bytes(S, LPP);
     auto kern = qr_kernel<LPP, false>;
     int grid = 0;

@@ -1872,10 +1872,7 @@ int dcpse_vjp_positions(dcpse_plan_t* P, const double* d_pos, const double* d_ep
             return rc;
         P->vjp_batch = a.scratch_particles;
     }
-    cudaError_t e = vjp_entries(a, *P->htab, P->stream);
-    if (e == cudaErrorInvalidConfiguration)
-        return fail(DCPSE_ERR_CAPACITY, "position VJP: the QR work space of this lane grouping exceeds shared memory");
-    DCPSE_CK(e);
+    DCPSE_CK(vjp_entries(a, *P->htab, P->stream));
     DCPSE_CK(vjp_gather(P->t_row, P->t_idx, n, P->dim, P->gentry, d_grad, P->stream));
     return DCPSE_OK;
 }
@@ -2164,17 +2161,15 @@ int apply_terms(dcpse_plan_t* P, const int* terms, int count, const double* d_f,
     };
     for (int i = 0; i < count;) {
         const double *K[kTermsFused], *eip[kTermsFused];
-        double* out[kTermsFused];
         const unsigned ord = order(terms[i]);
         int m = 0;
         for (; m < kTermsFused && i + m < count && order(terms[i + m]) % 2 == ord % 2; ++m) {
             const int t = terms[i + m];
             K[m] = P->k_term + (size_t)t * P->nnz;
             eip[m] = P->eip_group + (size_t)P->term_group[t] * P->n;
-            out[m] = d_out;
         }
         P->tstart(DCPSE_K_APPLY_TERM);
-        cudaError_t e = apply_terms_f64(P->n, P->rowptr, P->cols, m, K, eip, out, i > 0, ord, d_f, P->stream);
+        cudaError_t e = apply_terms_f64(P->n, P->rowptr, P->cols, m, K, eip, d_out, i > 0, ord, d_f, P->stream);
         P->tstop(DCPSE_K_APPLY_TERM);
         DCPSE_CK(e);
         i += m;

@@ -199,12 +199,11 @@ bool assembly_uses_tc(const AsmTables& h, int flags, int maxk);
 
 
 // ----------------------------------------------------------------- apply --
-// Terms in the reference's order: out[t] = (accumulate, or an earlier term with
-// the same out: out +) (sum_q (f_q + s f_p) K[t]_pq) eip[t]_p, s = -1 for even
-// order, else 1.
+// Terms in the reference's order, summed from the first on: out = (accumulate:
+// out +) sum_t (sum_q (f_q + s f_p) K[t]_pq) eip[t]_p, s = -1 for even order, else 1.
 constexpr int kTermsFused = 3;
 cudaError_t apply_terms_f64(int64_t n, const int64_t* rowptr, const int32_t* cols, int nterms, const double* const* K,
-                            const double* const* eip, double* const* out, int accumulate, unsigned order,
+                            const double* const* eip, double* out, int accumulate, unsigned order,
                             const double* f, cudaStream_t s);
 // (hi, lo) float pair of f[i * stride], i < n
 cudaError_t split_f64(const double* f, int64_t n, float2* f2, cudaStream_t s, int64_t stride = 1);
