@@ -181,6 +181,12 @@ struct CudaRt {
     static Error free(void* p) { return cudaFree(p); }
     static Error device(int* dev) { return cudaGetDevice(dev); }
     static void clear_error() { cudaGetLastError(); }
+    // this thread's captures let allocations and releases pass meanwhile
+    struct Relaxed {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+        ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    };
 };
 typedef DevicePoolT<CudaRt> DevicePool;
 
@@ -999,6 +1005,7 @@ int dcpse_plan_create(dcpse_plan_t** plan, int dim, int n_outputs, const int* te
 
 int dcpse_plan_destroy(dcpse_plan_t* P) {
     if (!P) return DCPSE_OK;
+    CudaRt::Relaxed relaxed;  // (a capture of this thread is no reason to end it)
     if (P->stream) cudaStreamSynchronize(P->stream);
     P->free_all();
     pool().wait();

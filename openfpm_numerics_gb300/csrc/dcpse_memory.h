@@ -14,7 +14,9 @@
 // itself, of a block of one byte: 2.2 us on an idle GPU with its cudaMalloc.  A
 // cudaDeviceSynchronize (0.6 us) is invalid while any stream of the device is
 // captured and ends that capture, also one of another thread in thread-local
-// mode, where cudaMalloc and cudaFree are allowed.
+// mode, where cudaMalloc and cudaFree are allowed.  Inside the wait and a release
+// they are allowed in captures of any mode, this thread's too: a plan that is
+// destroyed meanwhile (by a garbage collector, say) does not end them.
 //
 // Rt: the runtime's calls (CudaRt, or a fake in the host tests).
 #pragma once
@@ -92,9 +94,12 @@ public:
             std::lock_guard<std::mutex> lock(m_);
             stamp = stamp_;
         }
-        void* p = nullptr;
-        e = Rt::malloc(&p, 1);
-        if (e == Rt::ok) e = Rt::free(p);
+        {
+            typename Rt::Relaxed relaxed;
+            void* p = nullptr;
+            e = Rt::malloc(&p, 1);
+            if (e == Rt::ok) e = Rt::free(p);
+        }
         if (e == Rt::ok)
             noted([&] { synced_[dev] = std::max(synced_[dev], stamp); });
         else
@@ -121,6 +126,7 @@ public:
             blocks.swap(free_);
             cached_ = 0;
         }
+        typename Rt::Relaxed relaxed;
         for (auto& f : blocks) Rt::free(f.second.first);  // (any device's: pointers are unified)
     }
 

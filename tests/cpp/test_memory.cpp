@@ -27,11 +27,17 @@ struct Fake {
     static size_t used, limit;
     static int dev, last_error, frees;
     static bool refuse;                     // as under a global-mode capture
+    static bool broken;                     // no allocation at all
+    static thread_local bool relaxed;
+    struct Relaxed {
+        Relaxed() { relaxed = true; }
+        ~Relaxed() { relaxed = false; }
+    };
     static uintptr_t next;
     static int malloc(void** p, size_t bytes) {
         std::lock_guard<std::mutex> lock(m);
         *p = nullptr;
-        if (refuse) return last_error = 900;
+        if (broken || (refuse && !relaxed)) return last_error = 900;
         if (bytes > limit - used) return last_error = no_memory;
         used += bytes;
         *p = reinterpret_cast<void*>(next);
@@ -41,7 +47,7 @@ struct Fake {
     }
     static int free(void* p) {
         std::lock_guard<std::mutex> lock(m);
-        if (refuse) return last_error = 900;
+        if (refuse && !relaxed) return last_error = 900;
         auto it = blocks.find(p);
         if (it == blocks.end()) return last_error = 1;
         used -= it->second;
@@ -59,7 +65,8 @@ std::mutex Fake::m;
 std::map<void*, size_t> Fake::blocks;
 size_t Fake::used = 0, Fake::limit = ~size_t(0) / 2;
 int Fake::dev = 0, Fake::last_error = 0, Fake::frees = 0;
-bool Fake::refuse = false;
+bool Fake::refuse = false, Fake::broken = false;
+thread_local bool Fake::relaxed = false;
 uintptr_t Fake::next = 4096;
 
 typedef dcpse::DevicePoolT<Fake> Pool;
@@ -95,10 +102,21 @@ int main() {
         // no wait to be had: no block that may be in use is handed out, and no
         // error stays behind for the next launch to find
         pool.free(c);
-        Fake::refuse = true;
+        Fake::broken = true;
         CHECK(pool.wait() != 0 && Fake::last_error == 0);
         CHECK(pool.alloc(&a, 140000) != 0 && a == nullptr);
+        Fake::broken = false;
+        // under a capture the wait passes, a new allocation is refused as it was
+        CHECK(pool.alloc(&c, 5000) == 0);
+        pool.free(c);
+        Fake::refuse = true;
+        CHECK(pool.alloc(&a, 5000) == 0 && a == c);
+        CHECK(pool.alloc(&b, 700000) != 0 && b == nullptr);
+        pool.free(a);
+        pool.release();
+        CHECK(Fake::blocks.empty());
         Fake::refuse = false;
+        Fake::clear_error();
         // sizes that no device has are refused (and end: doubling a unit up to
         // them would wrap around)
         Fake::limit = size_t(1) << 40;

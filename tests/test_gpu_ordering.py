@@ -235,6 +235,29 @@ def test_position_vjp_beside_a_pending_assembly(cuda):
     plan.close()
 
 
+def test_plans_destroyed_inside_a_capture(cuda):
+    """Plans that end while this thread captures, the last one too, leave the
+    capture alone."""
+    pos, h = W.lattice(20, 2, jitter=0.1, seed=87)
+    p = torch.tensor(pos, device="cuda")
+    plans = []
+    for _ in range(2):
+        plans.append(DcpsePlan(2, [[(1, 0)]], stream=torch.cuda.Stream()))
+        plans[-1].build_neighbors(p, 3.1 * h)
+        plans[-1].assemble(p, FAST64)
+    x, y = torch.ones(100, device="cuda"), torch.zeros(100, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y.add_(x)
+        for plan in plans:
+            plan.close()
+        y.mul_(2.0)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, 2.0 * x)
+
+
 def test_released_memory_can_be_given_back(cuda):
     keep = DcpsePlan(2, [[(1, 0)]])
     pos, h = W.lattice(48, 3, jitter=0.1, seed=86)
