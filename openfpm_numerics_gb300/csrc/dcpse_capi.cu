@@ -461,6 +461,18 @@ struct dcpse_plan_s {
         dfree(nc.base);
         dfree(nc.flag);
     }
+    KeptForGraphs narrow_kept;  // sell_narrow
+    // the layout's 16-bit columns for a call on st
+    NarrowCols narrow_for(cudaStream_t st) {
+        if (sell_narrow.d) narrow_kept.used(capturing(st));
+        return sell_narrow;
+    }
+    // sell_narrow given up for room (false: there is none, or a graph may read it)
+    bool drop_narrow() {
+        const bool had = sell_narrow.d && narrow_kept.may_go();
+        if (had) free_narrow(sell_narrow);
+        return had;
+    }
     float* sell_w = nullptr;
     void* sell_r = nullptr;  // bf16 residuals on the same layout (with r16)
     float* sell_r32 = nullptr;  // FP32 residuals on the same layout (with r32: the weight pairs)
@@ -500,6 +512,7 @@ struct dcpse_plan_s {
         dfree(sell_off);
         dfree(sell_cols);
         free_narrow(sell_narrow);
+        narrow_kept = {};
         sell_total = 0;
     }
     void free_assembly() {
@@ -1933,7 +1946,7 @@ int dcpse_rk4_gs_stage(dcpse_plan_t* P, int stage, int precision, const void* Yu
                 a.srow = P->sell_row;
                 a.soff = P->sell_off;
                 a.scols = P->sell_cols;
-                a.narrow = P->sell_narrow;
+                a.narrow = P->narrow_for(P->stream);
                 a.sw = P->sell_w;
             }
         }
@@ -2308,11 +2321,7 @@ cudaError_t spare_or(T*& live, T*& spare, size_t count) {
 extern "C++" template <typename Alloc, typename Fill, typename Release>
 int sell_stream(dcpse_plan_t* P, const char* what, Alloc alloc, Fill fill, Release release) {
     // (rather without the 16-bit columns than without the weights)
-    cudaError_t e = with_room<CudaRt>(alloc, [&] {
-        const bool had = P->sell_narrow.d != nullptr;
-        dcpse_plan_s::free_narrow(P->sell_narrow);
-        return had;
-    });
+    cudaError_t e = with_room<CudaRt>(alloc, [&] { return P->drop_narrow(); });
     if (e == cudaSuccess) e = fill();
     if (e == cudaSuccess) e = cudaStreamSynchronize(P->stream);
     if (e == cudaSuccess) return DCPSE_OK;
@@ -2476,7 +2485,7 @@ int apply_f32_rows(dcpse_plan_t* P, int precision, double* d_out, int64_t r0, in
         sa.srow = P->sell_row;
         sa.off = P->sell_off;
         sa.cols = P->sell_cols;
-        sa.narrow = P->sell_narrow;
+        sa.narrow = P->narrow_for(st);
         sa.w = P->sell_w;
         sa.r = resid ? static_cast<const __nv_bfloat16*>(P->sell_r) : nullptr;
         sa.r32 = pair ? P->sell_r32 : nullptr;
@@ -3057,7 +3066,7 @@ int dcpse_p2p(dcpse_plan_t* P, const double* d_f_support, int ncomp, double* d_o
                     sa.srow = P->sell_row;
                     sa.off = P->sell_off;
                     sa.cols = P->sell_cols;
-                    sa.narrow = P->sell_narrow;
+                    sa.narrow = P->narrow_for(P->stream);
                     sa.w = P->sell_w;
                     sa.total = P->sell_total;
                     sa.f2 = P->f2;

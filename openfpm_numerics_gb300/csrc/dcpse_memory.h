@@ -209,4 +209,16 @@ typename Rt::Error with_less(Int& count, Int least, Alloc alloc) {
     }
 }
 
+// Whether an optional buffer may be given up for room: not once a call that was
+// captured has read it, since the graph keeps its address and may run at any time
+// while the plan's layout lives.
+class KeptForGraphs {
+public:
+    void used(bool capturing) { kept_ = kept_ || capturing; }
+    bool may_go() const { return !kept_; }
+
+private:
+    bool kept_ = false;
+};
+
 }  // namespace dcpse

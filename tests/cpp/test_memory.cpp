@@ -180,6 +180,33 @@ int main() {
         Fake::limit = ~size_t(0) / 2;
     }
     {
+        // what a captured call has read is not given up for room
+        Pool pool;
+        void *extra, *p;
+        dcpse::KeptForGraphs kept;
+        auto room = [&] {
+            const bool had = extra && kept.may_go();
+            if (had) pool.free(extra);
+            if (had) extra = nullptr;
+            return had;
+        };
+        auto want = [&] { return pool.alloc(&p, 900000); };
+        for (bool captured : {true, false}) {
+            Fake::limit = Fake::used + (size_t(1) << 20);
+            CHECK(pool.alloc(&extra, 500000) == 0);
+            kept = {};
+            kept.used(false);
+            kept.used(captured);
+            kept.used(false);
+            CHECK(dcpse::with_room<Fake>(want, room) == (captured ? Fake::no_memory : 0));
+            CHECK((extra != nullptr) == captured);
+            Fake::clear_error();
+            pool.free(captured ? extra : p);
+            pool.release();
+        }
+        Fake::limit = ~size_t(0) / 2;
+    }
+    {
         // threads: no two owners of a block at a time
         Pool pool;
         std::mutex m;
