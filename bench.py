@@ -509,7 +509,9 @@ def run_ours(args):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "traffic": traffic, "peak_source": peak_kind,
                          "kernel": kname,
-                         "algorithmic_bytes_per_launch": bytes_apply, "kernel_ms": t_kernel * 1e3},
+                         "algorithmic_bytes_per_launch": bytes_apply, "kernel_ms": t_kernel * 1e3,
+                         # (the algorithmic bytes count 4-byte columns; the kernel reads 2-byte ones)
+                         "traffic_frac": traffic / t_kernel / 1e9 / hbm if traffic else None},
             "e2e": {"value": job_value(world, N, NOUT, t_e2e), "unit": UNIT, "h2d_bytes_per_step": N * 8,
                     "d2h_bytes_per_step": NOUT * N * 8, "ms_per_step": t_e2e * 1e3,
                     "api": "dcpse_apply_batched_host"},
@@ -940,7 +942,11 @@ def gray_scott_run(args):
            "ms_per_step_graph": t_fwd,
            "roofline": {"bound": "hbm", "algorithmic_bytes_per_step": step_bytes,
                         "achieved_gbs": step_bytes / t_fwd / 1e6, "peak_gbs": hbm,
-                        "frac": step_bytes / t_fwd / 1e6 / hbm, "peak_source": peak_kind}, "backward_window_steps": window, "checkpoint_every": every,
+                        "frac": step_bytes / t_fwd / 1e6 / hbm, "peak_source": peak_kind,
+                        # with the 2-byte columns that the stages read (and their bases, one per 128
+                        # entries) in the place of the 4-byte ones
+                        "frac_16bit_columns": (step_bytes - 4 * nnz * (2 - 4 / 128)) / t_fwd / 1e6 / hbm},
+           "backward_window_steps": window, "checkpoint_every": every,
            "backward_ms": t_bwd, "backward_ms_per_step": t_bwd / window,
            "v_final_mean": float(gs.v.mean()), "grad_v_norm": float(vb.norm()),
            "finite": bool(torch.isfinite(gs.v).all() and torch.isfinite(vb).all())}
